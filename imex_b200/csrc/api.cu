@@ -68,11 +68,13 @@ void prof_harvest(imex_ctx* ctx) {
   ctx->prof_pending.clear();
 }
 
-// EOS iteration-cap flags of the two kernel translation units
+// EOS iteration-cap flags of the three kernel translation units
 imex_status eos_flag_stage(imex_ctx* ctx, int* flag, bool reset);
 imex_status eos_flag_solve(imex_ctx* ctx, int* flag, bool reset);
 imex_status eos_flag_stage_enqueue(imex_ctx* ctx, int* host_flag);
 imex_status eos_flag_solve_enqueue(imex_ctx* ctx, int* host_flag);
+imex_status eos_flag_march_enqueue(imex_ctx* ctx, int* host_flag);
+imex_status eos_flag_march_clear(imex_ctx* ctx);
 
 namespace {
 
@@ -183,14 +185,19 @@ imex_status device_status(imex_ctx* ctx, bool with_scalars = false) {
   if (e != cudaSuccess) return cuda_check(ctx, e, "status readback");
   imex_status q = eos_flag_stage_enqueue(ctx, &flags[0]);
   if (q == IMEX_OK) q = eos_flag_solve_enqueue(ctx, &flags[1]);
+  if (q == IMEX_OK) q = eos_flag_march_enqueue(ctx, &flags[2]);
   if (q != IMEX_OK) return q;
   e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return cuda_check(ctx, e, "status readback");
   int s = ctx->h_st->status;
   int f1 = flags[0], f2 = flags[1];
+  const int f3 = flags[2];
   if (f1) eos_flag_stage(ctx, &f1, true);  // clears it
   if (f2) eos_flag_solve(ctx, &f2, true);
-  if ((f1 || f2) && s < IMEX_ERR_EOS) s = IMEX_ERR_EOS;
+  if (f3) eos_flag_march_clear(ctx);
+  if ((f1 || f2 || f3) && s < IMEX_ERR_EOS) s = IMEX_ERR_EOS;
+  // a solve gave up waiting: its arrival counter and epoch no longer agree
+  if (s == IMEX_ERR_SYNC) cudaMemsetAsync(ctx->sync, 0, sizeof(SyncState), ctx->stream);
   if (s != IMEX_OK) {
     int zero = 0;
     cudaMemcpyAsync(&ctx->st->status, &zero, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
@@ -452,7 +459,7 @@ imex_status imex_create(const imex_config* cfg, int nx, int ny, imex_ctx** out) 
   A_(hh, N); A_(eta, N); A_(vscale, N); A_(tdiag, N); A_(vdiag, N); A_(rv, 3 * N);
   A_(irho, N);
   A_(pb, N); A_(pp, N); A_(pf, N); A_(pg, N); A_(pdp, N);
-  A_(mx, 3 * N); A_(mb, 3 * N);
+  A_(mx, 4 * N); A_(mb, 3 * N);
   if (!cfg->GLF) {
     A_(lvm, 4 * N); A_(lvp, 4 * N);
   }

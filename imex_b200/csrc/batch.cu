@@ -25,6 +25,7 @@
 
 #include "imex_internal.h"
 #include "launch.cuh"
+#include "march_host.h"
 
 struct imex_batch {
   std::vector<imex_ctx*> members;
@@ -551,8 +552,8 @@ imex_status imex_batch_autotune(imex_batch* b, int trial_steps, imex_batch_tunin
   // FP64 GMRES needs many Krylov steps: time both
   const int solves0 = c0->cfg.mixed_solves;
   const int mag = IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B;
-  // the tile shape matters for the B-form solve of the fast arithmetic, the one with choices
-  const bool tiles = c0->P.magfield != IMEX_PotentialA && c0->P.fast;
+  // the tile shape matters for the tile kernels' B-form solve of the fast arithmetic, the one with choices
+  const bool tiles = c0->P.magfield != IMEX_PotentialA && c0->P.fast && !march::supports(c0, IMEX_OP_MAGNETIC_B);
   struct Choice {
     int streams, restart, solves, tile;
   };

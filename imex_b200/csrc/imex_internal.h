@@ -92,12 +92,16 @@ struct ProfRec {
   double bytes;
 };
 
+constexpr int kMaxBlocks = 256;  // blocks of one row-marching solve (one per SM)
 // Grid-barrier and reduction workspace of the persistent solver kernels.
 struct SyncState {
   unsigned long long count;  // barrier arrivals since the launch started (monotonic, 64-bit: never wraps)
   int abort;
   int pad1;
   long long wait_cycles;  // bound of any single barrier wait, in SM clock cycles
+  // pass ends of the row-marching kernels (march.cuh): arrivals so far, over all launches; their
+  // number when the next launch starts; the mark of a launch that gave up, if any
+  unsigned long long arrivals, epoch, abort_at;
 };
 
 }  // namespace imex
@@ -132,7 +136,8 @@ struct imex_ctx {
   // operator's and the pressure operator's, built before their solves (k_local_visc)
   double *lvm = nullptr, *lvp = nullptr;
   double *pb = nullptr, *pp = nullptr, *pf = nullptr, *pg = nullptr, *pdp = nullptr;  // pressure vectors
-  double *mx = nullptr, *mb = nullptr;  // magnetic solution / rhs (3 planes each)
+  double* mb = nullptr;  // magnetic rhs (3 planes)
+  double* mx = nullptr;  // one-component solves: 1 / diagonal, right and upper face weights, a second 1 / diagonal
   double *chit = nullptr, *Epp = nullptr, *Et = nullptr;
   double* bline = nullptr;  // storage of the boundary lines
   imex::BoundaryLines bl{};

@@ -1,0 +1,57 @@
+// The row-marching solves of the ideal gas (pressure), the energy formula and the magnetic
+// systems, and the choice between them and the tile kernels.  Multiply-adds are contracted in
+// this file (build.py): a solve's rounding stays below its tolerance either way.
+#include "march_solve.cuh"
+
+namespace imex {
+namespace march {
+
+// The solves that run here: the fast arithmetic (the exact one keeps the reference's operation
+// order, which the face forms do not), global dissipation (the energy operator has none) and,
+// in the A form, periodic boundaries (an open tile extrapolates A past the edge).  The other
+// configurations keep the tile kernels.
+bool supports(const imex_ctx* ctx, int op) {
+  const DevParams& P = ctx->P;
+  if (!P.fast) return false;
+  if (op == IMEX_OP_ENERGY) return true;
+  if (op == IMEX_OP_MAGNETIC_A) return P.GLF && !P.xclamp && !P.yclamp;
+  return P.GLF != 0;
+}
+imex_status gmres_solve(imex_ctx* ctx, int op, int fam, double* x, const double* b, const Scratch* scratch) {
+  const bool rk = ctx->P.eos_type != IMEX_IDEAL_GAS;
+  if (op == IMEX_OP_PRESSURE_L || op == IMEX_OP_PRESSURE_J) {
+    const bool jac = op == IMEX_OP_PRESSURE_J;
+    return rk ? gmres_solve_rk(ctx, jac, fam, x, b, scratch)
+              : solve<PressureRow<double, false>>(ctx, jac, fam, IMEX_MIXED_PRESSURE, x, b, scratch);
+  }
+  if (op == IMEX_OP_ENERGY) return solve<EnergyRow<double>>(ctx, false, fam, IMEX_MIXED_PRESSURE, x, b, scratch);
+  if (op == IMEX_OP_MAGNETIC_B)
+    return solve<MagBRow<double>>(ctx, false, fam, IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B, x, b, scratch);
+  return solve<MagARow<double>>(ctx, false, fam, IMEX_MIXED_MAGNETIC, x, b, scratch);
+}
+imex_status newton_solve(imex_ctx* ctx, double* p, const double* b, int keys) {
+  if (ctx->P.eos_type != IMEX_IDEAL_GAS) return newton_solve_rk(ctx, p, b, keys);
+  return is_mixed(ctx, IMEX_MIXED_PRESSURE) ? newton_one<float, false>(ctx, p, b, keys)
+                                            : newton_one<double, false>(ctx, p, b, keys);
+}
+imex_status batch_build(BatchSolvePlan* plan, const std::vector<imex_ctx*>& members, int op, bool nested) {
+  imex_ctx* c0 = members[0];
+  if (op == IMEX_OP_MAGNETIC_A)
+    return add_solves<MagARow<double>>(plan, members, IMEX_MIXED_MAGNETIC, F_GMRES_MAG_A, magnetic_system);
+  if (op == IMEX_OP_MAGNETIC_B)
+    return add_solves<MagBRow<double>>(plan, members, IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B, F_GMRES_MAG_B,
+                                       magnetic_system);
+  if (op == IMEX_OP_ENERGY)
+    return add_solves<EnergyRow<double>>(plan, members, IMEX_MIXED_PRESSURE, F_GMRES_ENERGY, energy_system);
+  if (!nested)
+    return add_solves<PressureRow<double, false>>(plan, members, IMEX_MIXED_PRESSURE, F_NEWTON, pressure_system);
+  if (c0->P.eos_type != IMEX_IDEAL_GAS) return batch_newton_rk(plan, members);
+  return is_mixed(c0, IMEX_MIXED_PRESSURE) ? add_newtons<float, false>(plan, members)
+                                           : add_newtons<double, false>(plan, members);
+}
+size_t scratch_partials(imex_ctx* ctx) {
+  return (size_t)2 * (ctx->num_sms < kMaxBlocks ? ctx->num_sms : kMaxBlocks) * kSlots;
+}
+
+}  // namespace march
+}  // namespace imex

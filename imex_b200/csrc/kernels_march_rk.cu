@@ -1,0 +1,36 @@
+// The row-marching pressure solves of the Redlich-Kwong gas.  Multiply-adds stay uncontracted
+// here: the Newton's slope is a difference of the EOS over 2e-8, which amplifies the last ulp
+// of the EOS iterations, so they keep the reference's rounding.
+#include "march_solve.cuh"
+
+namespace imex {
+namespace march {
+
+imex_status gmres_solve_rk(imex_ctx* ctx, bool jac, int fam, double* x, const double* b, const Scratch* scratch) {
+  return solve<PressureRow<double, true>>(ctx, jac, fam, IMEX_MIXED_PRESSURE, x, b, scratch);
+}
+imex_status newton_solve_rk(imex_ctx* ctx, double* p, const double* b, int keys) {
+  return is_mixed(ctx, IMEX_MIXED_PRESSURE) ? newton_one<float, true>(ctx, p, b, keys)
+                                            : newton_one<double, true>(ctx, p, b, keys);
+}
+imex_status batch_newton_rk(BatchSolvePlan* plan, const std::vector<imex_ctx*>& members) {
+  return is_mixed(members[0], IMEX_MIXED_PRESSURE) ? add_newtons<float, true>(plan, members)
+                                                   : add_newtons<double, true>(plan, members);
+}
+
+}  // namespace march
+
+// this translation unit's EOS iteration-cap flag
+imex_status eos_flag_march_enqueue(imex_ctx* ctx, int* host_flag) {
+  return cuda_check(ctx, cudaMemcpyFromSymbolAsync(host_flag, d_eos_flag, sizeof(int), 0, cudaMemcpyDeviceToHost,
+                                                   ctx->stream),
+                    "eos flag");
+}
+imex_status eos_flag_march_clear(imex_ctx* ctx) {
+  static const int zero = 0;
+  cudaError_t e = cudaMemcpyToSymbolAsync(d_eos_flag, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  return cuda_check(ctx, e, "eos flag reset");
+}
+
+}  // namespace imex

@@ -24,6 +24,7 @@
 
 #include "cells.cuh"
 #include "launch.cuh"
+#include "march_host.h"
 
 namespace imex {
 namespace {
@@ -2551,7 +2552,13 @@ imex_status gmres_run(imex_ctx* ctx, const Op& o, int fam, double* x, const doub
   return s;
 }
 
+int gmres_family(int op) {
+  return op == IMEX_OP_MAGNETIC_B ? F_GMRES_MAG_B
+                                  : (op == IMEX_OP_MAGNETIC_A ? F_GMRES_MAG_A
+                                                              : (op == IMEX_OP_ENERGY ? F_GMRES_ENERGY : F_GMRES_PRES));
+}
 imex_status gmres_launch(imex_ctx* ctx, int op, double* x, const double* b) {
+  if (march::supports(ctx, op)) return march::gmres_solve(ctx, op, gmres_family(op), x, b);
   if (op == IMEX_OP_PRESSURE_L || op == IMEX_OP_PRESSURE_J) {
     PressureOp o = make_pressure_op(ctx);
     o.jac = op == IMEX_OP_PRESSURE_J;
@@ -2634,10 +2641,58 @@ imex_status gmres_noalloc_op(imex_ctx* ctx, const Op& o, int fam, double* x, con
   return cuda_check(ctx, e, "imex_gmres_noalloc: solve");
 }
 
+// The same for the solves of the row-marching kernels:
+//   barrier state | partial sums | V | AV | x, b staging (host only)
+imex_status gmres_noalloc_march(imex_ctx* ctx, int op, double* x, const double* b, unsigned char* base,
+                                size_t capacity) {
+  const size_t n = (op == IMEX_OP_MAGNETIC_B || op == IMEX_OP_MAGNETIC_A ? 3 : 1) * ctx->N;
+  const bool hx = !on_device(x), hb = !on_device(b);
+  size_t used = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = used;
+    used += (bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t o_sync = take(sizeof(SyncState));
+  const size_t o_part = take(march::scratch_partials(ctx) * sizeof(double));
+  const size_t o_V = take(((size_t)ctx->cfg.gmres_restart + 1) * n * sizeof(double));
+  const size_t o_AV = take(2 * n * sizeof(double));
+  const size_t o_x = hx ? take(n * sizeof(double)) : 0;
+  const size_t o_b = hb ? take(n * sizeof(double)) : 0;
+  if (used > capacity) {
+    char msg[256];
+    snprintf(msg, sizeof(msg),
+             "imex_gmres_noalloc: this solve needs %zu bytes of scratch (restart %d, %zu unknowns), "
+             "the static scratch holds %zu",
+             used, ctx->cfg.gmres_restart, n, capacity);
+    return set_error(ctx, IMEX_ERR_INVALID, msg);
+  }
+  march::Scratch w{};
+  w.sync = reinterpret_cast<SyncState*>(base + o_sync);
+  w.partial = reinterpret_cast<double*>(base + o_part);
+  w.V = reinterpret_cast<double*>(base + o_V);
+  w.AV = reinterpret_cast<double*>(base + o_AV);
+  double* xd = hx ? reinterpret_cast<double*>(base + o_x) : x;
+  const double* bd = hb ? reinterpret_cast<const double*>(base + o_b) : b;
+  cudaError_t e = cudaMemsetAsync(w.sync, 0, sizeof(SyncState), ctx->stream);
+  if (hx && e == cudaSuccess) e = cudaMemcpyAsync(xd, x, n * sizeof(double), cudaMemcpyDefault, ctx->stream);
+  if (hb && e == cudaSuccess) e = cudaMemcpyAsync((void*)bd, b, n * sizeof(double), cudaMemcpyDefault, ctx->stream);
+  if (e != cudaSuccess) return cuda_check(ctx, e, "imex_gmres_noalloc: vector upload");
+  imex_status s = march::gmres_solve(ctx, op, gmres_family(op), xd, bd, &w);
+  if (s != IMEX_OK) return s;
+  ctx->kernel_launches += ctx->prof_on ? 0 : 1;
+  if (hx) e = cudaMemcpyAsync(x, xd, n * sizeof(double), cudaMemcpyDefault, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  return cuda_check(ctx, e, "imex_gmres_noalloc: solve");
+}
+
 // keys: b is this context's pb just written by k_pressure_rhs into key slot `keys` - 1 (the
 // floor slope's inputs min b, max V); 0: the solve reduces them itself
 imex_status newton_launch(imex_ctx* ctx, double* p, const double* b, int keys = 0) {
   const DevParams& P = ctx->P;
+  if (march::supports(ctx, IMEX_OP_PRESSURE_L))
+    return !P.floor_on && P.eos_type == IMEX_IDEAL_GAS ? march::gmres_solve(ctx, IMEX_OP_PRESSURE_L, F_NEWTON, p, b)
+                                                       : march::newton_solve(ctx, p, b, keys);
   PressureOp o = make_pressure_op(ctx);
   if (!P.floor_on && P.eos_type == IMEX_IDEAL_GAS)  // a single linear GMRES with L (implicit_operators.cpp:664-668)
     return gmres_run(ctx, o, F_NEWTON, p, b, IMEX_MIXED_PRESSURE);
@@ -2841,7 +2896,11 @@ imex_status batch_solve_build(const std::vector<imex_ctx*>& members, int kind, B
   imex_ctx* c0 = members[0];
   const DevParams& P = c0->P;
   imex_status s;
-  if (kind == BATCH_MAGNETIC) {
+  const int op = kind == BATCH_MAGNETIC ? (P.magfield == IMEX_PotentialA ? IMEX_OP_MAGNETIC_A : IMEX_OP_MAGNETIC_B)
+                                        : (P.formula == IMEX_EnergyFormula ? IMEX_OP_ENERGY : IMEX_OP_PRESSURE_L);
+  if (march::supports(c0, op)) {  // members share the configuration
+    s = march::batch_build(plan, members, op, P.floor_on || P.eos_type != IMEX_IDEAL_GAS);
+  } else if (kind == BATCH_MAGNETIC) {
     auto sys = [](imex_ctx* m, double** x, const double** b) {
       int op;
       mag_system(m, &op, x, b);
@@ -3062,9 +3121,7 @@ imex_status run_pre_subsystem_pressure(imex_ctx* ctx, int rks) {
 imex_status run_pre_subsystem_energy(imex_ctx* ctx) {
   imex_status s;
   if ((s = energy_setup(ctx)) != IMEX_OK) return s;
-  if ((s = gmres_run(ctx, make_energy_op(ctx), F_GMRES_ENERGY, ctx->cons + 4 * ctx->N, ctx->pb,
-                     IMEX_MIXED_PRESSURE)) != IMEX_OK)
-    return s;
+  if ((s = gmres_launch(ctx, IMEX_OP_ENERGY, ctx->cons + 4 * ctx->N, ctx->pb)) != IMEX_OK) return s;
   return energy_momentum(ctx);
 }
 
@@ -3131,6 +3188,7 @@ imex_status run_gmres(imex_ctx* ctx, int op, double* x, const double* b) { retur
 
 imex_status run_gmres_noalloc(imex_ctx* ctx, int op, double* x, const double* b, unsigned char* base,
                               size_t capacity) {
+  if (march::supports(ctx, op)) return gmres_noalloc_march(ctx, op, x, b, base, capacity);
   if (op == IMEX_OP_PRESSURE_L || op == IMEX_OP_PRESSURE_J) {
     PressureOp o = make_pressure_op(ctx);
     o.jac = op == IMEX_OP_PRESSURE_J;

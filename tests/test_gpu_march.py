@@ -1,0 +1,117 @@
+"""The solves of the row-marching kernels (imex_b200/csrc/march_solve.cuh) at the sizes where
+their cut of the grid can go wrong: grids narrower than a strip (62 columns of a one-component
+vector, 30 and 28 of the B and A forms), one column past it, runs cut short at the last row, and
+enough tasks for several blocks; periodic and transmissive; FP64 and mixed; conjugate gradients
+and GMRES through their slot limits.
+
+Each solve's right-hand side is the operator (imex_apply_operator, which test_gpu_parity.py pins
+to the oracle) applied to a known vector of size one.  The error of the solution is the stopping
+tolerance, 1e-13 relative plus 1e-13 absolute in the preconditioned residual, times the
+condition number, below 1e3 for these steps (the diagonals lie between 1 and about 30): 1e-10 with
+the vector's norm.  The mixed form stops at mixed_outer_tol = 1e-10: 1e-7."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import imex_b200 as ix
+from conftest import rel
+from imex_b200.problems import open_blast, random_field, vortex, vortex_sheet
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(4, 4), (5, 9), (28, 7), (29, 4), (30, 6), (31, 5), (61, 8), (62, 5), (63, 4), (125, 7), (4, 131), (130, 71)]
+B_FORM = dict(recon="VanLeer", magfield="StaggerCT", GMREStol=1e-13)
+A_FORM = dict(recon="WENO5", magfield="PotentialA", GMREStol=1e-13)
+ENERGY = dict(recon="Minmod", magfield="StaggerCT", formula="EnergyFormula", GMREStol=1e-13)
+OPS = [("pressure_L", B_FORM, "vortex"), ("pressure_J", B_FORM, "vortex"), ("magnetic_B", B_FORM, "vortex"),
+       ("magnetic_A", A_FORM, "sheet"), ("energy", ENERGY, "vortex"), ("pressure_L", B_FORM, "blast"),
+       ("magnetic_B", B_FORM, "blast"), ("energy", ENERGY, "blast")]
+
+
+def _solver(kind, nx, ny, settings):
+    prob = {"vortex": vortex, "sheet": vortex_sheet, "blast": open_blast}[kind](nx, ny)
+    sv = ix.Solver.for_problem(prob, 2, settings)
+    for name in ("Qe", "Qs"):  # stage buffers of a state with variation in every plane
+        sv.set_buffer(name, sv.cons())
+    sv.set_scalars(vx_max=0.8, vy_max=0.9, B_max_x=0.7, B_max_y=0.6)
+    return sv, prob
+
+
+def _known(sv, op, seed=3):
+    n = sv.nx * sv.ny * (3 if op.startswith("magnetic") else 1)
+    return np.random.default_rng(seed).standard_normal(n)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("op,settings,kind", OPS)
+def test_march_solves_recover_a_known_vector(op, settings, kind, precision):
+    for nx, ny in SIZES:
+        sv, prob = _solver(kind, nx, ny, dict(settings, precision=precision, mixed_solves=7))
+        sv.prepare_operator(op, 2.0 * min(prob.dx, prob.dy))
+        if op == "pressure_J":  # some floored cells, whose slope is Mbig
+            sv.set_newton_state(np.where(np.arange(sv.N) % 7 == 3, -1.0, 1.0), 50.0)
+        x = _known(sv, op)
+        got, st = sv.gmres(op, np.zeros_like(x), sv.apply_operator(op, x))
+        assert st["status"] == 0
+        assert rel(got, x) <= (1e-10 if precision == "fp64" else 1e-7), (nx, ny, rel(got, x))
+        sv.close()
+
+
+@pytest.mark.parametrize("restart", [1, 2, 3, 25, 30])
+@pytest.mark.parametrize("op,settings,kind", [OPS[0], OPS[2], OPS[3], OPS[4]])
+def test_march_solves_with_few_and_many_slots(op, settings, kind, restart):
+    """Restarted GMRES, and conjugate gradients that fill their residual slots many times."""
+    sv, prob = _solver(kind, 63, 41, dict(settings, gmres_restart=restart))
+    sv.prepare_operator(op, 2.0 * min(prob.dx, prob.dy))
+    x = _known(sv, op)
+    got, st = sv.gmres(op, np.zeros_like(x), sv.apply_operator(op, x))
+    assert st["status"] == 0 and rel(got, x) <= 1e-10, (st, rel(got, x))
+    sv.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(5, 9), (63, 4), (130, 71)])
+@pytest.mark.parametrize("eos", ["IDEAL_GAS", "REDLICH_KWONG"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_march_newton_matches_the_tile_kernels(nx, ny, eos, precision):
+    """The nested Newton against the exact arithmetic's (the tile kernels) on a right-hand side
+    that floors some cells.  Both stop at a residual of 1e-8 of the first plus 1e-8; the Newton
+    converges quadratically, so the iterates agree to about the square of that: 1e-9."""
+    n = min(nx, ny)
+    res = []
+    for arith in ("exact", "fast"):
+        sv = ix.Solver.for_problem(vortex(nx, ny), 2, dict(B_FORM, arith=arith, eos_type=eos, m_alfa=0.05, m_b=0.1,
+                                                           p_floor=0.05, theta=0.5, precision=precision))
+        for name in ("Qe", "Qs"):
+            sv.set_buffer(name, sv.cons())
+        sv.set_scalars(vx_max=0.8, vy_max=0.9)
+        sv.prepare_operator("pressure_L", 0.5 * min(10.0 / nx, 10.0 / ny))
+        b = 1.5 * np.ones(sv.N)
+        b[:: 11] = 0.02
+        p, st = sv.nested_newton(np.full(sv.N, 0.9), b)
+        assert st["newton_iters"] >= 1
+        res.append(p)
+        sv.close()
+    assert rel(res[1], res[0]) <= 1e-9, (n, rel(res[1], res[0]))
+
+
+def test_march_falls_back_where_conjugate_gradients_break_down():
+    """A negative face weight (an operator that is not positive definite) hands the solve to GMRES."""
+    sv, prob = _solver("vortex", 63, 41, B_FORM)
+    sv.prepare_operator("pressure_J", 2.0 * min(prob.dx, prob.dy))
+    sv.set_newton_state(np.where(np.arange(sv.N) % 5 == 2, -1.0, 1.0), -40.0)  # slopes of both signs
+    x = _known(sv, "pressure_J")
+    got, st = sv.gmres("pressure_J", np.zeros_like(x), sv.apply_operator("pressure_J", x))
+    assert st["status"] == 0 and rel(got, x) <= 1e-8, (st, rel(got, x))
+    sv.close()
+
+
+def test_march_newton_is_bit_reproducible():
+    runs = []
+    for _ in range(2):
+        sv = ix.Solver.for_problem(random_field(65), 2, dict(recon="Minmod", magfield="StaggerCT", precision="mixed"))
+        for _ in range(2):
+            sv.step()
+        runs.append(sv.cons())
+        sv.close()
+    np.testing.assert_array_equal(runs[0], runs[1])
