@@ -802,7 +802,9 @@ struct Adj {
   size_t N;
   int R;
   double tol;
-  std::vector<void*> mem;
+  std::vector<void*> mem;  // this call's device memory
+  char* slab = nullptr;    // the call's checkpoints and outputs, one allocation cut up by amalloc
+  size_t slab_left = 0;
   std::vector<StageSnap> snap;
   DevScalars step_sc{};  // scalars after the prologue of the recomputed step
   double* step_prim;     // prim at the start of the recomputed step
@@ -821,19 +823,56 @@ struct Adj {
   double* hscal;             // pinned mirror of dscal
 };
 
+// bytes of a block of `count` doubles inside a slab
+size_t block_bytes(size_t count) { return ((count ? count : 1) * sizeof(double) + 255) & ~(size_t)255; }
 imex_status amalloc(Adj& W, double** p, size_t count) {
+  const size_t bytes = block_bytes(count);
+  if (bytes <= W.slab_left) {
+    *p = reinterpret_cast<double*>(W.slab);
+    W.slab += bytes;
+    W.slab_left -= bytes;
+    return IMEX_OK;
+  }
   void* q = nullptr;
-  cudaError_t e = cudaMalloc(&q, (count ? count : 1) * sizeof(double));
+  cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess) return cuda_check(W.ctx, e, "adjoint workspace");
   W.mem.push_back(q);
   *p = static_cast<double*>(q);
   return IMEX_OK;
 }
+// one allocation for `states` checkpoints (13 planes each) and the planes of the outputs
+imex_status state_slab(Adj& W, size_t states) {
+  const size_t N = W.N, bytes = states * (block_bytes(8 * N) + 2 * block_bytes(N) + block_bytes(3 * N)) +
+                                2 * block_bytes(8 * N) + block_bytes(N) + block_bytes(3 * N);
+  imex_ctx* ctx = W.ctx;
+  // a slab no larger than the workspace stays with the context too (an allocation and its release
+  // cost up to 100 ms on a busy host); a long run's checkpoints are given back with the call
+  const bool keep = bytes <= ctx->adj_ws_bytes;
+  void* q = nullptr;
+  if (keep && ctx->adj_slab && ctx->adj_slab_bytes >= bytes) {
+    q = ctx->adj_slab;
+  } else {
+    if (keep) {
+      cudaFree(ctx->adj_slab);
+      ctx->adj_slab = nullptr;
+      ctx->adj_slab_bytes = 0;
+    }
+    cudaError_t e = cudaMalloc(&q, bytes);
+    if (e != cudaSuccess) return cuda_check(ctx, e, "adjoint checkpoints");
+    if (keep) {
+      ctx->adj_slab = q;
+      ctx->adj_slab_bytes = bytes;
+    } else {
+      W.mem.push_back(q);
+    }
+  }
+  W.slab = static_cast<char*>(q);
+  W.slab_left = bytes;
+  return IMEX_OK;
+}
 void afree(Adj& W) {
   for (void* p : W.mem) cudaFree(p);
   W.mem.clear();
-  if (W.hscal) cudaFreeHost(W.hscal);
-  W.hscal = nullptr;
 }
 imex_status zero(Adj& W, double* p, size_t count) {
   return cuda_check(W.ctx, cudaMemsetAsync(p, 0, count * sizeof(double), W.ctx->stream), "adjoint clear");
@@ -855,12 +894,15 @@ imex_status put_sc(imex_ctx* ctx, const DevScalars& in) {
   return cuda_check(ctx, e, "adjoint scalars");
 }
 
+// The planes of the reverse sweep.  Their number depends on the context alone (grid, stages,
+// Energy_Modify), so the context keeps them from call to call, in one allocation, until it is
+// destroyed: with about 150 separate allocations per call a three-step product on 128^2 took
+// 48.6 ms (and 50 to 160 when the driver's allocator was slow), with these kept 29.3.
 imex_status workspace(Adj& W) {
   imex_ctx* ctx = W.ctx;
   const size_t N = W.N;
-  imex_status s = IMEX_OK;
-#define AL(p, c) \
-  if (s == IMEX_OK) s = amalloc(W, &(p), (c))
+  std::vector<std::pair<double**, size_t>> want;
+#define AL(p, c) want.push_back({&(p), (size_t)(c)})
   W.snap.resize(W.R);
   for (StageSnap& S : W.snap) {
     AL(S.Qe, 8 * N); AL(S.Qs, 8 * N); AL(S.bxQs, N); AL(S.byQs, N); AL(S.pe, N); AL(S.u1, 8 * N); AL(S.u2, 8 * N);
@@ -879,15 +921,27 @@ imex_status workspace(Adj& W) {
   AL(W.AT, 81 * N); AL(W.vdiag, N); AL(W.dscal, 16);
   if (ctx->P.Energy_Modify) AL(W.lbsave, 3 * N);
 #undef AL
-  if (s != IMEX_OK) return s;
-  void* q = nullptr;
-  cudaError_t e = cudaMalloc(&q, 8 * sizeof(unsigned long long));
-  if (e != cudaSuccess) return cuda_check(ctx, e, "adjoint workspace");
-  W.mem.push_back(q);
-  W.didx = static_cast<unsigned long long*>(q);
-  e = cudaMallocHost(&q, 16 * sizeof(double));
-  if (e != cudaSuccess) return cuda_check(ctx, e, "adjoint workspace");
-  W.hscal = static_cast<double*>(q);
+  double* idx = nullptr;
+  want.push_back({&idx, 8});
+  size_t bytes = 0;
+  for (const auto& q : want) bytes += block_bytes(q.second);
+  if (!ctx->adj_ws) {
+    cudaError_t e = cudaMalloc(&ctx->adj_ws, bytes);
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->adj_host, 16 * sizeof(double));
+    if (e != cudaSuccess) {
+      cudaFree(ctx->adj_ws);
+      ctx->adj_ws = nullptr;
+      return cuda_check(ctx, e, "adjoint workspace");
+    }
+    ctx->adj_ws_bytes = bytes;
+  }
+  char* at = static_cast<char*>(ctx->adj_ws);
+  for (const auto& q : want) {
+    *q.first = reinterpret_cast<double*>(at);
+    at += block_bytes(q.second);
+  }
+  W.didx = reinterpret_cast<unsigned long long*>(idx);
+  W.hscal = static_cast<double*>(ctx->adj_host);
   return IMEX_OK;
 }
 
@@ -1343,8 +1397,9 @@ imex_status adjoint_core(imex_ctx* ctx, const imex_adjoint_opts* o, const std::f
     if (t != IMEX_OK) return t;
     const int K = o->checkpoint_every, nsteps = o->nsteps;
     const int nseg = (nsteps + K - 1) / K;
-    std::vector<State> ck(nseg), seg(K);
+    std::vector<State> ck(nseg), seg(K < nsteps ? K : nsteps);
     State start{}, fin{};
+    if ((t = state_slab(W, ck.size() + seg.size() + 2)) != IMEX_OK) return t;
     if ((t = save_state(W, start)) != IMEX_OK) return t;
     for (int st = 0; st < nsteps; ++st) {
       if (st % K == 0 && (t = save_state(W, ck[st / K])) != IMEX_OK) return t;

@@ -511,6 +511,9 @@ imex_status imex_destroy(imex_ctx* ctx) {
   prof_harvest(ctx);
   for (cudaEvent_t e : ctx->prof_pool) cudaEventDestroy(e);
   for (void* p : ctx->allocations) cudaFree(p);
+  cudaFree(ctx->adj_ws);
+  cudaFree(ctx->adj_slab);
+  if (ctx->adj_host) cudaFreeHost(ctx->adj_host);
   if (ctx->h_sc) cudaFreeHost(ctx->h_sc);
   if (ctx->h_st) cudaFreeHost(ctx->h_st);
   if (ctx->h_red) cudaFreeHost(ctx->h_red);

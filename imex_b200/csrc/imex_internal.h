@@ -161,6 +161,9 @@ struct imex_ctx {
   double* red = nullptr;    // small reduction buffer (device)
   double* h_red = nullptr;  // pinned mirror
   std::vector<void*> allocations;
+  // the adjoint's workspace and checkpoints (adjoint.cu), and its pinned scalars
+  void *adj_ws = nullptr, *adj_slab = nullptr, *adj_host = nullptr;
+  size_t adj_ws_bytes = 0, adj_slab_bytes = 0;
   // live profile
   bool prof_on = false;
   std::vector<imex::ProfRec> prof_pending;
