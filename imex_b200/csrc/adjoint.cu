@@ -92,6 +92,9 @@ struct SeedLoad {
   }
 };
 
+// The passes over the inputs (L of them seeded at once) are independent, so they are spread
+// over blockIdx.y: a 128^2 grid has 128 blocks of cells, each with up to 28 passes one after
+// another otherwise.
 template <int L, class Fn>
 __global__ void __launch_bounds__(kAT) k_cell_vjp(DevParams P, CellVjp A, Fn fn) {
   __shared__ double s_acc[2];
@@ -117,7 +120,7 @@ __global__ void __launch_bounds__(kAT) k_cell_vjp(DevParams P, CellVjp A, Fn fn)
         nin += __popc(A.pmask[a]) * __popc(A.mask[a]);
       }
       const int ntot = nin + Fn::NS;
-      for (int q0 = 0; q0 < ntot; q0 += L) {
+      for (int q0 = blockIdx.y * L; q0 < ntot; q0 += gridDim.y * L) {
         ld.q0 = q0;
         Dual<L> sc[Fn::NS > 0 ? Fn::NS : 1];
 #pragma unroll
@@ -285,11 +288,23 @@ void cv_arr_planes(CellVjp& A, int a, const double* in, double* lam, unsigned pm
   A.pmask[a] = lam ? pmask : 0u;
   A.mask[a] = mask;
 }
+// Grid of a per-cell kernel whose `passes` independent passes may run in different blocks: as
+// many blocks of passes as fill the device eight blocks (32 warps) deep; on grids that do that by
+// themselves the passes stay in one thread, which then loads its cell once.  128^2: the cell
+// products 237 -> 125 us each.
+dim3 split_grid(const imex_ctx* ctx, int passes) {
+  const int gx = ablocks(ctx->P.N), want = 8 * (ctx->num_sms > 0 ? ctx->num_sms : 148);
+  int gy = (want + gx - 1) / gx;
+  if (gy > passes) gy = passes;
+  return dim3(gx, gy < 1 ? 1 : gy);
+}
 template <int L, class Fn>
 imex_status run_cell_vjp(imex_ctx* ctx, const CellVjp& A, Fn fn) {
   // unused arrays still need a readable base pointer for the value loads of the cell function
+  int inputs = Fn::NS;
+  for (int a = 0; a < kMaxArr; ++a) inputs += __builtin_popcount(A.pmask[a]) * __builtin_popcount(A.mask[a]);
   prof_begin(ctx);
-  k_cell_vjp<L, Fn><<<ablocks(ctx->P.N), kAT, 0, ctx->stream>>>(ctx->P, A, fn);
+  k_cell_vjp<L, Fn><<<split_grid(ctx, (inputs + L - 1) / L), kAT, 0, ctx->stream>>>(ctx->P, A, fn);
   ACHECK(ctx, "k_cell_vjp");
   prof_end(ctx, F_ADJ_CELLS, 0.0, 1);
   return IMEX_OK;
@@ -310,7 +325,11 @@ __global__ void __launch_bounds__(kAT) k_adj_flux(DevParams P, double h, double 
   if (n < N) {
     int i, j;
     cell_of(P, n, i, j);
-    for (int k = 0; k < 5; ++k) lam_Qs[k * N + n] += lam_u[k * N + n];
+    if (blockIdx.y == 0)
+      for (int k = 0; k < 5; ++k) lam_Qs[k * N + n] += lam_u[k * N + n];
+    // the face's direction and the block of seeded inputs may be spread over blockIdx.y: every
+    // entry of lam_w belongs to one face and one input
+    constexpr int NB = (NI + L - 1) / L;
     for (int dir = 0; dir < 2; ++dir) {
       const long long m = dir ? cid(P, i, j + 1) : cid(P, i + 1, j);
       const double d = dir ? P.dy : P.dx;
@@ -332,6 +351,7 @@ __global__ void __launch_bounds__(kAT) k_adj_flux(DevParams P, double h, double 
         qr[k] = kForm ? ucon[k * N + m] : 0.0;
       }
       for (int q0 = 0; q0 < NI; q0 += L) {
+        if ((dir * NB + q0 / L) % gridDim.y != blockIdx.y) continue;
         Dual<L> QL[8], QR[8], am(a_max);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -1246,7 +1266,7 @@ imex_status reverse_step(Adj& W) {
     if ((s = launch_reconstruct(ctx, false)) != IMEX_OK) return s;
     if ((s = copy(W, W.w, ctx->w, 32 * N)) != IMEX_OK) return s;
     prof_begin(ctx);
-    k_adj_flux<1><<<nb, kAT, 0, st>>>(P, h, S.sc.a_max, W.w, S.u2, W.l3, W.lw, W.l2, W.lQs, W.dscal + 0);
+    k_adj_flux<1><<<split_grid(ctx, 6), kAT, 0, st>>>(P, h, S.sc.a_max, W.w, S.u2, W.l3, W.lw, W.l2, W.lQs, W.dscal + 0);
     adj_recon(P, st, S.Qe, W.lw, W.lQe);
     ACHECK(ctx, "adjoint pressure flux");
     prof_end(ctx, F_ADJ_FLUX, 0.0, 2);
@@ -1296,7 +1316,7 @@ imex_status reverse_step(Adj& W) {
     // (9) convective flux: u1[0..4] = Qs - h div F(w(Qe), a_max)
     zero(W, W.lw, 32 * N);
     prof_begin(ctx);
-    k_adj_flux<0><<<nb, kAT, 0, st>>>(P, h, S.sc.a_max, W.w, S.u1, W.l1, W.lw, nullptr, W.lQs, W.dscal + 0);
+    k_adj_flux<0><<<split_grid(ctx, 6), kAT, 0, st>>>(P, h, S.sc.a_max, W.w, S.u1, W.l1, W.lw, nullptr, W.lQs, W.dscal + 0);
     adj_recon(P, st, S.Qe, W.lw, W.lQe);
     ACHECK(ctx, "adjoint convective flux");
     prof_end(ctx, F_ADJ_FLUX, 0.0, 2);

@@ -3282,7 +3282,7 @@ __global__ void k_adj_assemble_T(Op op, DevParams P, double* __restrict__ AT) {
   neighbours(P, n, nb);
   LocalTile<OD, D> t;
   local_fill(od, t, nb, nullptr, N);
-  for (int o = 0; o < 9; ++o) {
+  for (int o = blockIdx.y; o < 9; o += gridDim.y) {
     for (int kk = 0; kk < M; ++kk) t.s[kk * 9 + o].d[kk] = 1.0;
     D out[M];
     od.matvec(t, 0, 0, n, out);
@@ -3353,7 +3353,7 @@ __global__ void k_adj_coef_vjp(Op op, DevParams P, const double* __restrict__ x,
   local_fill(od, t, nb, x, N);
   double m[M];
   for (int k = 0; k < M; ++k) m[k] = mu[k * N + n];
-  for (int o = 0; o < 9; ++o) {
+  for (int o = blockIdx.y; o < 9; o += gridDim.y) {
     for (int q = 0; q < QT; ++q) t.c[q * 9 + o].d[q] = 1.0;
     D out[M];
     od.matvec(t, 0, 0, n, out);
@@ -3404,6 +3404,12 @@ __global__ void k_adj_visc_vjp(Op op, DevParams P, const double* __restrict__ x,
   }
 }
 
+// grid of the kernels that evaluate the operator once per neighbour: the nine evaluations go to
+// different blocks until the device is filled four blocks (32 warps) deep
+dim3 nine_grid(const imex_ctx* ctx) {
+  const int gx = blocks_for(ctx->P.N), gy = (4 * (ctx->num_sms > 0 ? ctx->num_sms : 148) + gx - 1) / gx;
+  return dim3(gx, gy < 1 ? 1 : (gy > 9 ? 9 : gy));
+}
 template <class Op>
 imex_status adj_op_dispatch(imex_ctx* ctx, const AdjOp& a, Op* out);
 template <>
@@ -3435,7 +3441,7 @@ imex_status adj_transpose_solve_op(imex_ctx* ctx, const AdjOp& a, double* AT, do
   const DevParams& P = ctx->P;
   const int nb = blocks_for(P.N);
   prof_begin(ctx);
-  k_adj_assemble_T<Op><<<nb, kThreads, 0, ctx->stream>>>(op, P, AT);
+  k_adj_assemble_T<Op><<<nine_grid(ctx), kThreads, 0, ctx->stream>>>(op, P, AT);
   LAUNCH_CHECK(ctx, "k_adj_assemble_T");
   prof_end(ctx, F_ADJ_ASSEMBLE, 0.0, 1);
   cudaError_t e = cudaMemsetAsync(mu, 0, (size_t)M * P.N * sizeof(double), ctx->stream);
@@ -3464,7 +3470,7 @@ imex_status adj_coef_vjp_op(imex_ctx* ctx, const AdjOp& a, const double* x, cons
   LamPlanes L{};
   for (int q = 0; q < Op::QT && q < 4; ++q) L.p[q] = lam_q[q];
   prof_begin(ctx);
-  k_adj_coef_vjp<Op><<<nb, kThreads, 0, ctx->stream>>>(op, P, x, mu, L);
+  k_adj_coef_vjp<Op><<<nine_grid(ctx), kThreads, 0, ctx->stream>>>(op, P, x, mu, L);
   LAUNCH_CHECK(ctx, "k_adj_coef_vjp");
   if (lam_visc) {
     k_adj_visc_vjp<Op><<<nb, kThreads, 0, ctx->stream>>>(op, P, x, mu, lam_visc);
