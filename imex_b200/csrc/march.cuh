@@ -30,11 +30,14 @@ struct Geom {
   int xclamp, yclamp;
   long long N;
 };
+// A clamped halo column is column nx - 1; lanes past it may hold any cell, and take different
+// ones (mirrored): asynchronous copies of one address by many lanes are served one after another,
+// which made the last strip of an open 700 x 450 grid, ten columns wide, 50 % slower.
 __device__ __forceinline__ int map_x(const Geom& G, int x) {
   if (x < 0) return G.xclamp ? 0 : x + G.nx;
-  if (x >= G.nx) {  // lanes past the last halo column may hold any cell
-    const int w = x - G.nx;
-    return G.xclamp || w >= G.nx ? G.nx - 1 : w;
+  if (x >= G.nx) {
+    const int w = x - G.nx, m = G.nx - 1 - w;
+    return G.xclamp || w >= G.nx ? (m > 0 ? m : 0) : w;
   }
   return x;
 }
@@ -128,7 +131,7 @@ struct PressureCoef {
 template <class T_, bool kRK>
 struct PressureRow : PressureCoef {
   using T = T_;
-  static constexpr int M = 1, H = 1, C = 2, kLag = 0, W = kRK ? 12 : 8, R = kRK ? 9 : 14, kAhead = 0;
+  static constexpr int M = 1, H = 1, C = 2, kLag = 0, W = kRK ? 12 : 8, R = kRK ? 9 : 14, kDots = 8, kAhead = 0;
   static constexpr bool kIsRK = kRK;
   static constexpr int kCoef = 2 + (kRK ? 2 : 0);  // planes read per application (+ vdiag in J mode)
   template <class U>
@@ -221,7 +224,7 @@ struct FaceCoef {
 template <class T_>
 struct FaceRow : FaceCoef {
   using T = T_;
-  static constexpr int M = 1, H = 1, C = 2, kLag = 0, W = 8, R = 14, kAhead = 0;
+  static constexpr int M = 1, H = 1, C = 2, kLag = 0, W = 8, R = 14, kDots = 8, kAhead = 0;
   static constexpr int kCoef = 3;
   __device__ __forceinline__ T slope(int o) const {
     if (p) return (T)(p[o] >= p_floor ? a : Mbig);
@@ -298,7 +301,7 @@ struct EnergyCoef {
 template <class T_>
 struct EnergyRow : EnergyCoef {
   using T = T_;
-  static constexpr int M = 1, H = 1, C = 2, kLag = 0, W = 8, R = 14, kAhead = 0;
+  static constexpr int M = 1, H = 1, C = 2, kLag = 0, W = 8, R = 14, kDots = 8, kAhead = 0;
   static constexpr bool kIsRK = false;
   static constexpr int kCoef = 1;
   template <class U>
@@ -371,7 +374,7 @@ struct MagBCoef {
 template <class T_>
 struct MagBRow : MagBCoef {
   using T = T_;
-  static constexpr int M = 3, H = 1, C = 1, kLag = 0, W = 8, R = 10, kAhead = 5;
+  static constexpr int M = 3, H = 1, C = 1, kLag = 0, W = 8, R = 8, kDots = 8, kAhead = 5;
   static constexpr int kCoef = 4;
   template <class U>
   __device__ __forceinline__ MagBRow<U> as() const {
@@ -487,7 +490,7 @@ struct MagACoef {
 template <class T_>
 struct MagARow : MagACoef {
   using T = T_;
-  static constexpr int M = 3, H = 2, C = 1, kLag = 1, W = 12, R = 5, kAhead = 0;
+  static constexpr int M = 3, H = 2, C = 1, kLag = 1, W = 12, R = 4, kDots = 8, kAhead = 0;
   static constexpr int kCoef = 4;
   template <class U>
   __device__ __forceinline__ MagARow<U> as() const {

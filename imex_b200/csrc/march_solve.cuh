@@ -15,8 +15,8 @@
 // on middle grids, and on small grids the pass end.  The tile kernels (kernels_solve.cu), which
 // keep the configurations these do not take, stage 32 x 16 tiles in shared memory with two or
 // three block barriers per tile and were latency bound at 24-33 % of the issue slots.  Measured
-// against them, us per solve: A form 1024^2 429 -> 287, 2048^2 1520 -> 945; B form 768^2 (Krylov
-// spaces of 25) 2533 -> 2137, 320^2 296 -> 232; nested Newton 64^2 131 -> 90, 700 x 450 348 ->
+// against them, us per solve: A form 1024^2 429 -> 277, 2048^2 1520 -> 919; B form 768^2 (Krylov
+// spaces of 25) 2533 -> 1966, open 700 x 450 900 -> 553, 320^2 296 -> 210; nested Newton 64^2 131 -> 90, 700 x 450 348 ->
 // 148, 1024^2 326 -> 169, 2048^2 1189 -> 670, Redlich-Kwong 768^2 689 -> 411; one pressure solve
 // of 75 steps on 513 x 400 1609 -> 620.
 #pragma once
@@ -62,7 +62,7 @@ template <class Op, class TS>
 struct Ring {
   static constexpr int M = Op::M, C = Op::C;
   static constexpr int kSlots_ = Op::H + 2, kVec = Op::R * (int)(8 / sizeof(TS));
-  static constexpr int kReg = Op::R < 8 ? Op::R : 8;  // vectors whose dot products a lane sums in registers
+  static constexpr int kReg = Op::R < Op::kDots ? Op::R : Op::kDots;  // dot products that a lane sums in registers
   static constexpr int kBytes = kSlots_ * Op::R * M * C * 32 * 8;  // per warp
   TS* p;  // the lane's first element
   __device__ __forceinline__ TS* at(int it, int i) const { return p + ((it % kSlots_) * kVec + i) * M * C * 32; }
@@ -217,14 +217,27 @@ __device__ __forceinline__ void ring_copy(const Ring<Op, TS>& R, const Work<TS>&
   constexpr int M = Op::M, C = Op::C;
   const long long N = g.G.N;
   const int nr = n < R.kVec ? n : R.kVec;
+  if (nr <= 0) return;
   TS* d = R.at(it, 0);
-#pragma unroll 4
-  for (int i = 0; i < nr; ++i, d += M * C * 32) {
-    const TS* p = basis<Op>(g, i);
+  const TS* p[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    p[c] = g.V0 + off[c];
+#pragma unroll
+    for (int m = 0; m < M; ++m) copy_async(d + (m * C + c) * 32, p[c] + m * N);
+    p[c] = g.V + M * N + off[c];
+  }
+  // from the second vector on the planes follow one another
+#pragma unroll 3
+  for (int i = 1; i < nr; ++i) {
+    d += M * C * 32;
 #pragma unroll
     for (int m = 0; m < M; ++m)
 #pragma unroll
-      for (int c = 0; c < C; ++c) copy_async(d + (m * C + c) * 32, p + m * N + off[c]);
+      for (int c = 0; c < C; ++c) {
+        copy_async(d + (m * C + c) * 32, p[c]);
+        p[c] += N;
+      }
   }
 }
 // the vectors past the ring in a row, K of them from i on, in registers
@@ -263,7 +276,7 @@ __device__ __forceinline__ void ring_add(const Ring<Op, TS>& R, const Work<TS>& 
   constexpr int M = Op::M, C = Op::C, kReg = Ring<Op, TS>::kReg, kVec = Ring<Op, TS>::kVec;
   constexpr bool kAhead = Op::kAhead > 0;
   Rest<Op, TS> rest;
-  if (kAhead) rest.load(g, kVec, n, off);
+  if (kAhead && n > kVec) rest.load(g, kVec, n, off);
   copy_wait();
   const TS* d = R.at(it, 0);
 #pragma unroll
@@ -284,7 +297,7 @@ __device__ __forceinline__ void ring_add(const Ring<Op, TS>& R, const Work<TS>& 
 #pragma unroll
       for (int c = 0; c < C; ++c) v[m][c] = fma(a, (double)d[((i * M + m) * C + c) * 32], v[m][c]);
   }
-  if (kAhead) rest.add(wt, kVec, n, v);
+  if (kAhead && n > kVec) rest.add(wt, kVec, n, v);
 #pragma unroll 1
   for (int i = kVec + (kAhead ? Rest<Op, TS>::K : 0); i < n; i += Rest<Op, TS>::K) {
     rest.load(g, i, n, off);
@@ -409,7 +422,7 @@ struct ArnoldiFill {
   const TS* AVj;
   int n;  // basis vectors: j + 1
   __device__ __forceinline__ void ahead(const int (&eo)[C]) const {
-    if (Op::kAhead > 0) dr.load(g, Ring<Op, TS>::kVec, n, eo);
+    if (Op::kAhead > 0 && n > Ring<Op, TS>::kVec) dr.load(g, Ring<Op, TS>::kVec, n, eo);
   }
   struct Buf {
     TS h[M][C];
@@ -520,7 +533,7 @@ __device__ __forceinline__ bool pass_arnoldi(const Op& op, const Work<TS>& g, Sm
     if (i <= j) {
       double q[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) q[u] = i + u < kReg ? dv[i + u] : 0.0;
+      for (int u = 0; u < 4; ++u) q[u] = i + u < kReg ? dv[i + u < kReg ? i + u : 0] : 0.0;
       const double r = warp_sum4(q);
       if ((lane & 7) == 0 && i + (lane >> 3) < kReg) S.acc[warp][i + (lane >> 3)] = r;
     }
