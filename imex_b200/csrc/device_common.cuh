@@ -263,82 +263,65 @@ __device__ __forceinline__ void load_cell(const double* __restrict__ a, long lon
 // left and right face values of the cell, reconstruction.cpp:38-266.
 // kFast (imex_config.arith = fast): WENO5 forms its normalised weights with one division per
 // face (w_k / sum w = d_k P_k / sum_i d_i P_i, P_k the product of the other two smoothness
-// terms) and its polynomials with fused multiply-adds; VanLeer takes 1 / (1 + r) once.
+// terms) from the differences of its stencil, with fused multiply-adds; VanLeer takes 1 / (1 + r) once.
+// The fast WENO5 of one variable along one direction, before the normalisation: the face
+// values are wL = u0 + nL / (6 dL) and wR = u0 + nR / (6 dR).  Everything is formed from the
+// four differences of the stencil: the polynomials enter as 6 (q_k - u0), the smoothness
+// measures as 4 e_k, the linear weights as (3, 6, 1) (the normalisation takes the common
+// factors out), which is 46 operations for both faces where the polynomials of the values
+// themselves took 71, and a constant field gives its value exactly.
 template <class S>
-__device__ inline void weno5_fast(S um2, S um1, S u0, S up1, S up2, S& wL, S& wR) {
-  const S a0 = um2 - 2 * um1 + u0, b0 = fma(S(3), u0, um2 - 4 * um1);
-  const S a1 = um1 - 2 * u0 + up1, b1 = um1 - up1;
-  const S a2 = u0 - 2 * up1 + up2, b2 = fma(S(3), u0, up2 - 4 * up1);
-  const S e0 = fma(13.0 / 12.0 * a0, a0, fma(0.25 * b0, b0, S(1e-6)));
-  const S e1 = fma(13.0 / 12.0 * a1, a1, fma(0.25 * b1, b1, S(1e-6)));
-  const S e2 = fma(13.0 / 12.0 * a2, a2, fma(0.25 * b2, b2, S(1e-6)));
+__device__ __forceinline__ void weno5_parts(S um2, S um1, S u0, S up1, S up2, S& nL, S& dL, S& nR, S& dR) {
+  const S d0 = um1 - um2, d1 = u0 - um1, d2 = up1 - u0, d3 = up2 - up1;
+  const S a0 = d1 - d0, a1 = d2 - d1, a2 = d3 - d2;
+  const S b0 = fma(S(2.0), d1, a0), b1 = d1 + d2, b2 = fma(S(-2.0), d2, a2);
+  const S e0 = fma(13.0 / 3.0 * a0, a0, fma(b0, b0, S(4e-6)));
+  const S e1 = fma(13.0 / 3.0 * a1, a1, fma(b1, b1, S(4e-6)));
+  const S e2 = fma(13.0 / 3.0 * a2, a2, fma(b2, b2, S(4e-6)));
   const S s0 = e0 * e0, s1 = e1 * e1, s2 = e2 * e2;
-  const S t0 = s1 * s2, t1 = s0 * s2, t2 = s0 * s1;
+  const S t0 = s1 * s2, t1 = 6.0 * (s0 * s2), t2 = s0 * s1;
   {
-    const S q0 = fma(-1.0 / 6.0, um2, fma(5.0 / 6.0, um1, 1.0 / 3.0 * u0));
-    const S q1 = fma(1.0 / 3.0, um1, fma(5.0 / 6.0, u0, -1.0 / 6.0 * up1));
-    const S q2 = fma(11.0 / 6.0, u0, fma(-7.0 / 6.0, up1, 1.0 / 3.0 * up2));
-    const S a = 0.3 * t0, b = 0.6 * t1, c = 0.1 * t2;
-    wL = fma(a, q0, fma(b, q1, c * q2)) / (a + b + c);
+    const S a = 3.0 * t0;
+    const S q0 = fma(S(-4.0), d1, d0), q1 = fma(S(-2.0), d1, -d2), q2 = fma(S(2.0), a2, -3.0 * d2);
+    nL = fma(a, q0, fma(t1, q1, t2 * q2));
+    dL = a + t1 + t2;
   }
   {
-    const S q0 = fma(1.0 / 3.0, um2, fma(-7.0 / 6.0, um1, 11.0 / 6.0 * u0));
-    const S q1 = fma(-1.0 / 6.0, um1, fma(5.0 / 6.0, u0, 1.0 / 3.0 * up1));
-    const S q2 = fma(1.0 / 3.0, u0, fma(5.0 / 6.0, up1, -1.0 / 6.0 * up2));
-    const S a = 0.1 * t0, b = 0.6 * t1, c = 0.3 * t2;
-    wR = fma(a, q0, fma(b, q1, c * q2)) / (a + b + c);
+    const S c = 3.0 * t2;
+    const S q0 = fma(S(2.0), a0, 3.0 * d1), q1 = fma(S(2.0), d2, d1), q2 = fma(S(4.0), d2, -d3);
+    nR = fma(t0, q0, fma(t1, q1, c * q2));
+    dR = t0 + t1 + c;
   }
 }
-// The fast WENO5 of one cell in x and y at once: the same weights and polynomials as
-// weno5_fast, with the four normalisations (1 / (a + b + c) of each face) taken from one
-// division of their product (plus nine multiplications) instead of four divisions.  Where
-// that product leaves the normal double range (smoothness sums beyond ~1e75 or below ~1e-75)
-// the four divisions are taken as in weno5_fast.
+template <class S>
+__device__ inline void weno5_fast(S um2, S um1, S u0, S up1, S up2, S& wL, S& wR) {
+  S nL, dL, nR, dR;
+  weno5_parts(um2, um1, u0, up1, up2, nL, dL, nR, dR);
+  wL = u0 + nL / (6.0 * dL);
+  wR = u0 + nR / (6.0 * dR);
+}
+// The fast WENO5 of one cell in x and y at once: the four normalisations (1 / d of each face)
+// taken from one division of their product (plus nine multiplications) instead of four
+// divisions.  Where that product leaves the normal double range (smoothness sums beyond ~1e75
+// or below ~1e-75) the four divisions are taken as in weno5_fast.
 __device__ inline void weno5_fast_xy(const double (&v)[5], const double (&u)[5], double& xl, double& xr, double& yl,
                                      double& yr) {
-  double nL[2], dL[2], nR[2], dR[2];
-#pragma unroll
-  for (int d = 0; d < 2; ++d) {
-    const double um2 = d ? u[0] : v[0], um1 = d ? u[1] : v[1], u0 = d ? u[2] : v[2];
-    const double up1 = d ? u[3] : v[3], up2 = d ? u[4] : v[4];
-    const double a0 = um2 - 2 * um1 + u0, b0 = fma(3.0, u0, um2 - 4 * um1);
-    const double a1 = um1 - 2 * u0 + up1, b1 = um1 - up1;
-    const double a2 = u0 - 2 * up1 + up2, b2 = fma(3.0, u0, up2 - 4 * up1);
-    const double e0 = fma(13.0 / 12.0 * a0, a0, fma(0.25 * b0, b0, 1e-6));
-    const double e1 = fma(13.0 / 12.0 * a1, a1, fma(0.25 * b1, b1, 1e-6));
-    const double e2 = fma(13.0 / 12.0 * a2, a2, fma(0.25 * b2, b2, 1e-6));
-    const double s0 = e0 * e0, s1 = e1 * e1, s2 = e2 * e2;
-    const double t0 = s1 * s2, t1 = s0 * s2, t2 = s0 * s1;
-    {
-      const double q0 = fma(-1.0 / 6.0, um2, fma(5.0 / 6.0, um1, 1.0 / 3.0 * u0));
-      const double q1 = fma(1.0 / 3.0, um1, fma(5.0 / 6.0, u0, -1.0 / 6.0 * up1));
-      const double q2 = fma(11.0 / 6.0, u0, fma(-7.0 / 6.0, up1, 1.0 / 3.0 * up2));
-      const double a = 0.3 * t0, b = 0.6 * t1, c = 0.1 * t2;
-      nL[d] = fma(a, q0, fma(b, q1, c * q2));
-      dL[d] = a + b + c;
-    }
-    {
-      const double q0 = fma(1.0 / 3.0, um2, fma(-7.0 / 6.0, um1, 11.0 / 6.0 * u0));
-      const double q1 = fma(-1.0 / 6.0, um1, fma(5.0 / 6.0, u0, 1.0 / 3.0 * up1));
-      const double q2 = fma(1.0 / 3.0, u0, fma(5.0 / 6.0, up1, -1.0 / 6.0 * up2));
-      const double a = 0.1 * t0, b = 0.6 * t1, c = 0.3 * t2;
-      nR[d] = fma(a, q0, fma(b, q1, c * q2));
-      dR[d] = a + b + c;
-    }
-  }
-  const double px = dL[0] * dR[0], py = dL[1] * dR[1], pp = px * py;
+  double nxl, dxl, nxr, dxr, nyl, dyl, nyr, dyr;
+  weno5_parts(v[0], v[1], v[2], v[3], v[4], nxl, dxl, nxr, dxr);
+  weno5_parts(u[0], u[1], u[2], u[3], u[4], nyl, dyl, nyr, dyr);
+  const double px = dxl * dxr, py = dyl * dyr, pp = px * py;
   if (pp > 1e-300 && pp < 1e300) {
-    const double r = 1.0 / pp;
-    const double rx = py * r, ry = px * r;  // 1 / px and 1 / py
-    xl = nL[0] * (dR[0] * rx);
-    xr = nR[0] * (dL[0] * rx);
-    yl = nL[1] * (dR[1] * ry);
-    yr = nR[1] * (dL[1] * ry);
+    const double r = (1.0 / 6.0) / pp;
+    const double rx = py * r, ry = px * r;  // 1 / (6 px) and 1 / (6 py)
+    xl = fma(nxl, dxr * rx, v[2]);
+    xr = fma(nxr, dxl * rx, v[2]);
+    yl = fma(nyl, dyr * ry, u[2]);
+    yr = fma(nyr, dyl * ry, u[2]);
   } else {
-    xl = nL[0] / dL[0];
-    xr = nR[0] / dR[0];
-    yl = nL[1] / dL[1];
-    yr = nR[1] / dR[1];
+    xl = v[2] + nxl / (6.0 * dxl);
+    xr = v[2] + nxr / (6.0 * dxr);
+    yl = u[2] + nyl / (6.0 * dyl);
+    yr = u[2] + nyr / (6.0 * dyr);
   }
 }
 template <bool kFast = false, class S>

@@ -10,6 +10,8 @@
 // overlap another's arithmetic.
 #pragma once
 
+#include <type_traits>
+
 #include "cells.cuh"
 
 namespace imex {
@@ -147,9 +149,13 @@ struct PressureRow : PressureCoef {
     T vs[C], vd[C], id[C];
     T dg[C], kx[C], ky[C];  // from step: precP's diagonal less vd, the weights of the right and upper face
   };
-  struct State {
+  struct GeneralState {
     T x[C], h[C], e[C], gH[C], fH[C], fE[C];  // the row, and its lower face's mean and products
   };
+  struct FaceState {
+    T x[C], h[C], hS[C], sx[C], sy[C], f[C];  // the row, h below it, its halves of the face weights, the lower product
+  };
+  using State = typename std::conditional<kRK, GeneralState, FaceState>::type;
   __device__ __forceinline__ void load(const int (&o)[C], Row& r) const {
 #pragma unroll
     for (int c = 0; c < C; ++c) {
@@ -167,6 +173,46 @@ struct PressureRow : PressureCoef {
   }
   __device__ __forceinline__ void step(State& s, const T (&w)[M][C], const Row& n, Emit& em, T (&out)[M][C],
                                        T (&wc)[M][C]) const {
+    if constexpr (kRK) general(s, w, n, em, out, wc);
+    else faces(s, w, n, em, out, wc);
+  }
+  // the ideal gas: the slope factor is the constant a, so the two products of a face are one with
+  // the weight hh2 idx2 h + a h cvx e of the face means of h and e, which is the sum of a half from
+  // either cell: five exchanges between columns instead of six and half the products
+  __device__ __forceinline__ void faces(State& s, const T (&w)[M][C], const Row& n, Emit& em, T (&out)[M][C],
+                                        T (&wc)[M][C]) const {
+    const T hf = T(0.5), ax = hf * (T)(hh2 * idx2), bx = hf * (T)(a * h * cvx), ay = hf * (T)(hh2 * idy2),
+            by = hf * (T)(a * h * cvy);
+    T xE[C], hE[C], hW[C], sE[C], r[C], l[C];
+    right(s.x, xE);
+    right(s.h, hE);
+    left(s.h, hW);
+    right(s.sx, sE);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      em.kx[c] = s.sx[c] + sE[c];
+      r[c] = em.kx[c] * (xE[c] - s.x[c]);
+    }
+    left(r, l);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const T sy = ay * n.h[c] + by * n.e[c];
+      em.ky[c] = s.sy[c] + sy;
+      const T u = em.ky[c] * (w[0][c] - s.x[c]);
+      out[0][c] = em.vd[c] * s.x[c] - ((r[c] - l[c]) + (u - s.f[c]));
+      const T h2 = s.h[c] + s.h[c];
+      em.dg[c] = ax * (hE[c] + hW[c] + h2) + ay * (n.h[c] + s.hS[c] + h2);
+      wc[0][c] = s.x[c];
+      s.x[c] = w[0][c];
+      s.hS[c] = s.h[c];
+      s.h[c] = n.h[c];
+      s.sx[c] = ax * n.h[c] + bx * n.e[c];
+      s.sy[c] = sy;
+      s.f[c] = u;
+    }
+  }
+  __device__ __forceinline__ void general(State& s, const T (&w)[M][C], const Row& n, Emit& em, T (&out)[M][C],
+                                          T (&wc)[M][C]) const {
     const T hf = T(0.5);
     T xE[C], hE[C], eE[C], gR[C], vR[C], rH[C], rE[C], gL[C], lH[C], lE[C];
     right(s.x, xE);
@@ -191,8 +237,6 @@ struct PressureRow : PressureCoef {
       const T lap = (T)cvx * (rE[c] - lE[c]) + (T)cvy * (uE - s.fE[c]);
       out[0][c] = r - em.vs[c] * (T)h * lap;
       em.dg[c] = (T)hh2 * ((T)idx2 * (gR[c] + gL[c]) + (T)idy2 * (gU + s.gH[c]));
-      em.kx[c] = (T)(hh2 * idx2) * gR[c] + (T)(a * h * cvx) * vR[c];
-      em.ky[c] = (T)(hh2 * idy2) * gU + (T)(a * h * cvy) * vU;
       wc[0][c] = s.x[c];
       s.x[c] = w[0][c];
       s.h[c] = n.h[c];

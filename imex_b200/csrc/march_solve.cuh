@@ -316,7 +316,7 @@ struct IterateFill {
   const double* scale;  // the update's terms are multiplied by it (conjugate gradients), or null
   int na;               // terms of the pending update
   long long N;
-  static constexpr bool kScale = kSymmetric<Op>;
+  static constexpr bool kScale = kSymmetric<Op> || std::is_base_of<FaceCoef, Op>::value;
   struct Buf {
     double v[Op::M][Op::C], d[Op::M][Op::C], b[Op::M][Op::C], r[kRho ? Op::C : 1], f[kScale ? Op::C : 1];
   };
@@ -350,14 +350,14 @@ struct IterateFill {
   }
 };
 
-// rows of x with the right-hand side b of the completed row
-template <class Op>
+// rows of x with the right-hand side b of the completed row (and rho)
+template <class Op, bool kRho = false>
 struct RhsFill {
   __device__ __forceinline__ void ahead(const int (&)[Op::C]) const {}
-  const double *p, *b;
+  const double *p, *b, *rho;
   long long N;
   struct Buf {
-    double v[Op::M][Op::C], b[Op::M][Op::C];
+    double v[Op::M][Op::C], b[Op::M][Op::C], r[kRho ? Op::C : 1];
   };
   __device__ __forceinline__ void issue(int, const int (&off)[Op::C], const int (&eo)[Op::C], Buf& u) const {
 #pragma unroll
@@ -366,6 +366,7 @@ struct RhsFill {
       for (int c = 0; c < Op::C; ++c) {
         u.v[m][c] = p[m * N + off[c]];
         u.b[m][c] = b[m * N + eo[c]];
+        if (kRho) u.r[c] = __ldg(rho + eo[c]);
       }
   }
   template <class T>
@@ -554,7 +555,7 @@ __device__ __forceinline__ bool pass_residual(const Op& op, const Work<TS>& g, S
   const long long N = g.G.N;
   acc_clear(S);
   double rr = 0.0;
-  RhsFill<Op> fill{x, b, N};
+  RhsFill<Op> fill{x, b, nullptr, N};
   auto emit = [&](int, const int (&eo)[C], const bool (&own)[C], const T (&)[M][C], T (&out)[M][C],
                   const typename Op::Emit& em, const typename RhsFill<Op>::Buf& u) {
 #pragma unroll
@@ -954,7 +955,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
   int iters = 0, code = GM_MAXIT;
   const bool cg = kSym && g.kmax > 1;
   for (int outer = 0; outer < g.max_restarts; ++outer) {
-    bool ok;
+    bool ok = false;
     if constexpr (!kScalar<Op>) {
       ok = pass_residual<false>(op, g, S, y, x, b);
     } else {
@@ -1208,20 +1209,41 @@ __device__ __forceinline__ double rk_V(const DevParams& P, double rho, double p,
   slope = rho * (P.m_cv - 0.5 * U * rs / T) / (K + 0.5 * A * rs / T);
   return rho * (P.m_cv * T + U * rs);
 }
-template <class Op, class TS>
+// the residual pass's sums: |g|^2, |r0|^2, floored cells, smallest pressure
+struct NewtonSums {
+  double gg = 0.0, rr = 0.0, nf = 0.0, mn = INFINITY;
+  __device__ __forceinline__ void add(const DevParams& P, double gv, double r0, double pv) {
+    gg += gv * gv;
+    rr += r0 * r0;
+    if (pv < P.p_floor) nf += 1.0;
+    mn = fmin(mn, pv);
+  }
+  template <int W>
+  __device__ __forceinline__ bool end(Shared& S, Sync& y) {
+    double t[4] = {gg, rr, nf, 0.0};
+    const double s = warp_sum4(t);
+    mn = warp_min(mn);
+    const int lane = threadIdx.x & 31;
+    if ((lane & 7) == 0 && lane < 24) S.acc[threadIdx.x >> 5][lane >> 3] = s;
+    if (lane == 0) S.acc[threadIdx.x >> 5][3] = mn;
+    return pass_end<W>(y, S, 4, 8u);
+  }
+};
+// kFirst: the first residual pass of a Newton solve, which has no pending update and (ideal gas)
+// leaves the face weights
+template <bool kFirst, class Op, class TS>
 __device__ __forceinline__ bool pass_newton(const Op& op, const Work<TS>& g, const NewtonArgs& na, Smem<Op>& sm, Sync& y,
                                             const double* pc, double* pn, double Mbig, const double* scale, double* idg,
-                                            bool pending, bool dp_live, bool first, bool raw) {
+                                            bool pending, bool dp_live, bool raw) {
   constexpr int C = Op::C;
   constexpr bool kRK = Op::kIsRK;
   const DevParams& P = op.P;
   Shared& S = sm.S;
   acc_clear(S);
-  double gg = 0.0, rr = 0.0, nf = 0.0, mn = INFINITY;
-  IterateFill<Op, TS, kRK> fill{g,    S,    ring_of<Op, TS>(sm),      pc, dp_live ? na.dp : nullptr,
-                                na.b, na.rho, scale, pending ? S.nalpha : 0, 0};
+  NewtonSums sum;
+  using Fill = typename std::conditional<kFirst, RhsFill<Op, kRK>, IterateFill<Op, TS, kRK>>::type;
   auto emit = [&](int, const int (&eo)[C], const bool (&own)[C], const double (&wc)[1][C], double (&out)[1][C],
-                  const typename Op::Emit& em, const typename IterateFill<Op, TS, kRK>::Buf& u) {
+                  const typename Op::Emit& em, const typename Fill::Buf& u) {
 #pragma unroll
     for (int c = 0; c < C; ++c)
       if (own[c]) {
@@ -1248,27 +1270,66 @@ __device__ __forceinline__ bool pass_newton(const Op& op, const Work<TS>& g, con
           na.vdiag[eo[c]] = vs;
         }
         idg[eo[c]] = id;
-        if (first && !kRK) {
+        if (kFirst && !kRK) {
           op.kx[eo[c]] = em.kx[c];
           op.ky[eo[c]] = em.ky[c];
         }
         g.V0n[eo[c]] = (TS)(raw ? -gv : r0);
-        gg += gv * gv;
-        rr += r0 * r0;
-        if (pv < P.p_floor) nf += 1.0;
-        mn = fmin(mn, pv);
+        sum.add(P, gv, r0, pv);
       }
   };
-  for_tasks<Op::W>(g, [&](int task) { run_task<Op>(op, g.G, task, fill, emit); });
-  double t[4] = {gg, rr, nf, 0.0};
-  const double s = warp_sum4(t);
-  mn = warp_min(mn);
-  const int lane = threadIdx.x & 31;
-  if ((lane & 7) == 0 && lane < 24) S.acc[threadIdx.x >> 5][lane >> 3] = s;
-  if (lane == 0) S.acc[threadIdx.x >> 5][3] = mn;
+  if constexpr (kFirst) {
+    Fill fill{pc, na.b, na.rho, 0};
+    for_tasks<Op::W>(g, [&](int task) { run_task<Op>(op, g.G, task, fill, emit); });
+  } else {
+    Fill fill{g, S, ring_of<Op, TS>(sm), pc, dp_live ? na.dp : nullptr, na.b, na.rho, scale, pending ? S.nalpha : 0, 0};
+    for_tasks<Op::W>(g, [&](int task) { run_task<Op>(op, g.G, task, fill, emit); });
+  }
   count(g, S, 1 + (pending ? S.nalpha : 0),
-        Op::kCoef + (kRK ? 1 : 0) + 4 + (raw ? 0 : 2) + (first && !kRK ? 2 : 0) + (dp_live ? 1 : 0) + (scale ? 1 : 0));
-  return pass_end<Op::W>(y, S, 4, 8u);
+        Op::kCoef + (kRK ? 1 : 0) + 4 + (raw ? 0 : 2) + (kFirst && !kRK ? 2 : 0) + (dp_live ? 1 : 0) + (scale ? 1 : 0));
+  return sum.template end<Op::W>(S, y);
+}
+// The later residual passes of the ideal gas, while no cell of the iterate before was floored:
+// L p from the face weights that the first pass left (two exchanges between columns instead of
+// five, no means of h and e), and the preconditioner's diagonal from its reciprocal there, which
+// only a newly floored cell changes.
+template <class TS>
+__device__ __forceinline__ bool pass_newton_faces(const PressureRow<double, false>& op, const Work<TS>& g,
+                                                  const NewtonArgs& na, Smem<FaceRow<double>>& sm, Sync& y,
+                                                  const double* pc, double* pn, double Mbig, const double* scale,
+                                                  const double* id, double* idn, bool pending, bool dp_live) {
+  using Op = FaceRow<double>;
+  constexpr int C = Op::C;
+  const DevParams& P = op.P;
+  Shared& S = sm.S;
+  acc_clear(S);
+  NewtonSums sum;
+  Op f{};
+  f.kx = op.kx;
+  f.ky = op.ky;
+  f.idg = id;
+  f.a = op.a;
+  IterateFill<Op, TS> fill{g, S, ring_of<Op, TS>(sm), pc, dp_live ? na.dp : nullptr, na.b, na.rho, scale, pending ? S.nalpha : 0, 0};
+  auto emit = [&](int, const int (&eo)[C], const bool (&own)[C], const double (&wc)[1][C], double (&out)[1][C],
+                  const Op::Emit& em, const typename IterateFill<Op, TS>::Buf& u) {
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      if (own[c]) {
+        const double pv = wc[0][c];
+        double gv = out[0][c] - u.b[0][c], id = em.id[c];
+        if (P.floor_on && !(pv >= P.p_floor)) {
+          gv = out[0][c] - op.a * pv + fma(Mbig, pv - P.p_floor, op.a * P.p_floor) - u.b[0][c];
+          id = 1.0 / (Mbig + (1.0 / id - op.a));
+        }
+        pn[eo[c]] = pv;
+        idn[eo[c]] = id;
+        g.V0n[eo[c]] = (TS)-gv;
+        sum.add(P, gv, -gv * id, pv);
+      }
+  };
+  for_tasks<Op::W>(g, [&](int task) { run_task<Op>(f, g.G, task, fill, emit); });
+  count(g, S, 1 + (pending ? S.nalpha : 0), Op::kCoef + 4 + (dp_live ? 1 : 0));
+  return sum.template end<Op::W>(S, y);
 }
 template <class TS, bool kRK>
 __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<TS> g, const NewtonArgs& na,
@@ -1328,11 +1389,17 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   // the other (the slopes of floored cells change between Newton iterations)
   double *id = op.idg, *idn = kRK ? op.idg : na.idg2;
   bool pending = false, dp_live = false, scaled = false;
-  bool cg = !kRK && g.kmax > 1;
+  bool cg = !kRK && g.kmax > 1, faces = false;
+  Smem<FaceRow<double>>& sm_faces = reinterpret_cast<Smem<FaceRow<double>>&>(smd);
   int it, iters = 0, worst = GM_CONVERGED;
   for (it = 0; it < P.Pnewton_max; ++it) {
-    if (!pass_newton<L>(op, g, na, smd, y, pc, pn, Mbig, scaled ? id : nullptr, idn, pending, dp_live, it == 0, cg))
-      return GM_SYNC;
+    const double* scale = scaled ? id : nullptr;
+    bool ok = false;
+    if (it == 0) ok = pass_newton<true>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, pending, dp_live, cg);
+    else if (faces) {
+      if constexpr (!kRK) ok = pass_newton_faces(op, g, na, sm_faces, y, pc, pn, Mbig, scale, id, idn, pending, dp_live);
+    } else ok = pass_newton<false>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, pending, dp_live, cg);
+    if (!ok) return GM_SYNC;
     {
       double* q = id;
       id = idn;
@@ -1360,6 +1427,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       g.st->gmres_solves += 1;
       g.st->newton_iters += 1;
     }
+    faces = cg && S.red[2] == 0.0;
     if constexpr (!kRK) {
       // conjugate gradients take the slope of a cell from its pressure; without floored cells
       // every slope is the constant a and the passes read nothing
@@ -1389,7 +1457,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       }
       if (code == GM_BREAK) {
         // not positive definite: the update so far counts as this iteration's, GMRES takes the next
-        cg = false;
+        cg = faces = false;
         code = GM_CONVERGED;
       }
       for (int outer = 0; !scaled; ++outer) {
