@@ -75,6 +75,12 @@ __device__ __forceinline__ void copy_async(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// waits until at most n groups are in flight
+template <int n>
+__device__ __forceinline__ void copy_wait_but() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(n) : "memory");
+}
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <class Op>
@@ -726,10 +732,16 @@ __device__ __forceinline__ void apply_update(const Work<TS>& g, Shared& S, doubl
 // M^-1 sum_k c_k r_k with c_k = alpha_k + beta_{k+1} c_{k+1}, formed when the solve ends (or the
 // slots are full).  A non-positive curvature hands the solve to GMRES.
 template <bool kFirst, class Op, class TS>
-__device__ __forceinline__ bool pass_cg(const Op& op, const Work<TS>& g, Shared& S, Sync& y, int k, int par, double alpha,
-                                        double beta) {
+__device__ __forceinline__ bool pass_cg(const Op& op, const Work<TS>& g, Smem<Op>& sm, Sync& y, int k, int par,
+                                        double alpha, double beta) {
   using T = typename Op::T;
   constexpr int C = Op::C;
+  Shared& S = sm.S;
+  // rows on their way to the lane (its own columns): kStage - 1 ahead of the one in work
+  constexpr int kStage = 4, kRow = 6 * C * 32;
+  static_assert(kStage * kRow * 8 <= Ring<Op, double>::kBytes, "the stages live in the ring");
+  double* const stage = reinterpret_cast<double*>(sm.ring[threadIdx.x >> 5]);
+  auto stage_at = [&](int it) -> double* { return stage + (it & (kStage - 1)) * kRow; };
   const Geom& G = g.G;
   const int lane = threadIdx.x & 31;
   const TS* r0 = basis<Op>(g, k);
@@ -750,25 +762,24 @@ __device__ __forceinline__ bool pass_cg(const Op& op, const Work<TS>& g, Shared&
       xo[c] = map_x(G, x);
     }
     const int ya = seg * G.L, yb = ya + G.L < G.ny ? ya + G.L : G.ny, rows = yb - ya;
-    struct In {
-      TS r[C], w[C], s[C];
-      double id[C];
-      typename Op::Row k;
-      T vd[C];
-    } in;
-    int off[C];
+    // row `it` into its slot: kx, ky, id as doubles, then r, w, s
     auto issue = [&](int it) {
-      const int o = map_y(G, ya - 1 + it) * G.nx;
+      if (it < rows + 2) {
+        const int o = map_y(G, ya - 1 + it) * G.nx;
+        double* d = stage_at(it) + lane;
+        TS* t = reinterpret_cast<TS*>(stage_at(it) + 3 * C * 32) + lane;
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        off[c] = o + xo[c];
-        in.r[c] = r0[off[c]];
-        if (!kFirst) in.w[c] = w0[off[c]];
-        if (hist) in.s[c] = s0[off[c]];
-        in.id[c] = op.idg[off[c]];
-        in.vd[c] = op.slope(off[c]);
+        for (int c = 0; c < C; ++c) {
+          const int n = o + xo[c];
+          copy_async(d + c * 32, op.kx + n);
+          copy_async(d + (C + c) * 32, op.ky + n);
+          copy_async(d + (2 * C + c) * 32, op.idg + n);
+          copy_async(t + c * 32, r0 + n);
+          if (!kFirst) copy_async(t + (C + c) * 32, w0 + n);
+          if (hist) copy_async(t + (2 * C + c) * 32, s0 + n);
+        }
       }
-      op.load(off, in.k);
+      copy_commit();
     };
     typename Op::State st{};
     T vd[C];
@@ -778,14 +789,40 @@ __device__ __forceinline__ bool pass_cg(const Op& op, const Work<TS>& g, Shared&
       vd[c] = T(0);
       op_[c] = 0;
     }
-    issue(0);
+    __syncwarp();  // the slots of the task before are read
+#pragma unroll
+    for (int it = 0; it < kStage - 1; ++it) issue(it);
 #pragma unroll 1
     for (int it = 0; it < rows + 2; ++it) {
-      const In n = in;
+      struct {
+        TS r[C], w[C], s[C];
+        double id[C];
+        typename Op::Row k;
+        T vd[C];
+      } n;
+      const int o = map_y(G, ya - 1 + it) * G.nx;
       int on[C];
 #pragma unroll
-      for (int c = 0; c < C; ++c) on[c] = off[c];
-      if (it < rows + 1) issue(it + 1);
+      for (int c = 0; c < C; ++c) {
+        on[c] = o + xo[c];
+        n.vd[c] = op.slope(on[c]);
+      }
+      copy_wait_but<kStage - 2>();
+      {
+        const double* d = stage_at(it) + lane;
+        const TS* t = reinterpret_cast<const TS*>(stage_at(it) + 3 * C * 32) + lane;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          n.k.kx[c] = (T)d[c * 32];
+          n.k.ky[c] = (T)d[(C + c) * 32];
+          n.id[c] = d[(2 * C + c) * 32];
+          n.r[c] = t[c * 32];
+          if (!kFirst) n.w[c] = t[(C + c) * 32];
+          if (hist) n.s[c] = t[(2 * C + c) * 32];
+        }
+      }
+      __syncwarp();  // every lane has read the row before, whose slot the next copies take
+      issue(it + kStage - 1);
       T u[C], out[C];
 #pragma unroll
       for (int c = 0; c < C; ++c) {
@@ -846,14 +883,15 @@ __device__ __forceinline__ void cg_weights(Shared& S, int k) {
 // From r0 in V0 (not preconditioned).  On return the update M^-1 sum_i coef_i V_i of the last
 // slots waits in S; full slots were added to x before (x_live: x already holds a part).
 template <class Op, class TS>
-__device__ __forceinline__ int cg_solve(const Op& op, const Work<TS>& g, Shared& S, Sync& y, double tol_eff, double* x,
+__device__ __forceinline__ int cg_solve(const Op& op, const Work<TS>& g, Smem<Op>& sm, Sync& y, double tol_eff, double* x,
                                         bool& x_live, int& iters) {
+  Shared& S = sm.S;
   const int tid = threadIdx.x;
   int par = 0, k = 0, cycles = 0;
   __syncthreads();
   if (tid == 0) S.nalpha = 0;
   if (lead(g)) S.cycles += 1;
-  if (!pass_cg<true>(op, g, S, y, 0, par, 0.0, 0.0)) return GM_SYNC;
+  if (!pass_cg<true>(op, g, sm, y, 0, par, 0.0, 0.0)) return GM_SYNC;
   double gamma = S.red[0], alpha = gamma / S.red[1], beta = 0.0;
   if (!(gamma > 0.0) || !(alpha > 0.0) || !isfinite(alpha)) return GM_BREAK;
   for (;;) {
@@ -862,7 +900,7 @@ __device__ __forceinline__ int cg_solve(const Op& op, const Work<TS>& g, Shared&
       S.cgb[k] = beta;
     }
     par ^= 1;
-    if (!pass_cg<false>(op, g, S, y, k, par, alpha, beta)) return GM_SYNC;
+    if (!pass_cg<false>(op, g, sm, y, k, par, alpha, beta)) return GM_SYNC;
     ++iters;
     const double gn = S.red[0], delta = S.red[1], res = sqrt(S.red[2]);
     __syncthreads();
@@ -977,7 +1015,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
     if constexpr (kSym) {
       if (cg && outer == 0) {
         bool live = true;
-        code = cg_solve(kop, g, S, y, tol_eff, x, live, iters);
+        code = cg_solve(kop, g, sm, y, tol_eff, x, live, iters);
         scaled = true;
       }
     }
@@ -1123,7 +1161,7 @@ __device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, dou
     int c2 = GM_MAXIT;
     scaled = cg;
     if constexpr (kSymmetric<Op>) {  // one cycle, so x is not touched before the next sweep
-      if (cg) c2 = cg_solve(op32, g, S, y, g.tol * res + g.tol_abs, xc, x_live, iters);
+      if (cg) c2 = cg_solve(op32, g, sm, y, g.tol * res + g.tol_abs, xc, x_live, iters);
     }
     if (!scaled) {
       if (threadIdx.x == 0) S.gam[0] = res;
@@ -1453,7 +1491,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       __syncthreads();
       scaled = cg;
       if constexpr (!kRK) {
-        if (cg) code = cg_solve(J, g, S, y, tol_eff, na.dp, dp_live, iters);
+        if (cg) code = cg_solve(J, g, sm, y, tol_eff, na.dp, dp_live, iters);
       }
       if (code == GM_BREAK) {
         // not positive definite: the update so far counts as this iteration's, GMRES takes the next
