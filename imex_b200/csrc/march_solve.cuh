@@ -719,6 +719,57 @@ __device__ __forceinline__ void apply_update(const Work<TS>& g, Shared& S, doubl
   count(g, S, na * M, (zero ? 1 : 2) * M);
 }
 
+// A task's rows for passes of one halo row whose planes are copied into per-lane slots of shared
+// memory kStage - 1 rows ahead of the one in work (each lane copies and reads its own columns).
+// copy(it, c, n): asynchronous copies of cell n, column c, into the slot of iteration it.  The
+// caller loops over it < count(): wait(it, on) (row it, the cells on[], is in its slot), reads
+// the slot, next(it, copy), then works.
+template <int C, int kStage>
+struct StagedRows {
+  const Geom& G;
+  int xo[C], ya, rows;
+  bool own[C];
+  __device__ __forceinline__ StagedRows(const Geom& g, int task) : G(g) {
+    const int strip = task / G.nseg, seg = task - strip * G.nseg, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int q = lane + 32 * c, x = strip * G.wd + q - 1;
+      own[c] = q >= 1 && q < 1 + G.wd && x < G.nx;
+      xo[c] = map_x(G, x);
+    }
+    ya = seg * G.L;
+    rows = (ya + G.L < G.ny ? ya + G.L : G.ny) - ya;
+  }
+  __device__ __forceinline__ int count() const { return rows + 2; }
+  __device__ __forceinline__ bool inner(int it) const { return it >= 1 && it <= rows; }  // the task's own rows
+  template <class Copy>
+  __device__ __forceinline__ void issue(int it, Copy& copy) const {
+    if (it < rows + 2) {
+      const int o = map_y(G, ya - 1 + it) * G.nx;
+#pragma unroll
+      for (int c = 0; c < C; ++c) copy(it, c, o + xo[c]);
+    }
+    copy_commit();
+  }
+  template <class Copy>
+  __device__ __forceinline__ void start(Copy& copy) const {
+    __syncwarp();  // the slots of the task before are read
+#pragma unroll
+    for (int it = 0; it < kStage - 1; ++it) issue(it, copy);
+  }
+  __device__ __forceinline__ void wait(int it, int (&on)[C]) const {
+    const int o = map_y(G, ya - 1 + it) * G.nx;
+#pragma unroll
+    for (int c = 0; c < C; ++c) on[c] = o + xo[c];
+    copy_wait_but<kStage - 2>();
+  }
+  template <class Copy>
+  __device__ __forceinline__ void next(int it, Copy& copy) const {
+    __syncwarp();  // every lane has read the row before, whose slot the next copies take
+    issue(it + kStage - 1, copy);
+  }
+};
+
 // ------------------------------------------------------------------ conjugate gradients
 // The symmetric one-component systems (FaceRow) take preconditioned conjugate gradients in the
 // form with one reduction per step (Chronopoulos and Gear, s-step iterative methods for
@@ -1369,7 +1420,184 @@ __device__ __forceinline__ bool pass_newton_faces(const PressureRow<double, fals
   count(g, S, 1 + (pending ? S.nalpha : 0), Op::kCoef + 4 + (dp_live ? 1 : 0));
   return sum.template end<Op::W>(S, y);
 }
-template <class TS, bool kRK>
+// V_mod and V_slope of the ideal gas where the pressure is below the floor (config.hpp:206-239)
+__device__ __forceinline__ double floored_V(const PressureRow<double, false>& op, double Mbig, double pv) {
+  return fma(Mbig, pv - op.P.p_floor, op.a * op.P.p_floor);
+}
+// The two residual passes of the ideal gas for tasks of many rows, with their rows copied ahead
+// through the slots of the ring: 1024^2 and 2048^2 gain 6 and 8 % of the Newton solve, tasks of
+// a few rows lose to the longer prologue (700 x 450, 4 rows a task, 4 %).
+// The first residual pass of the ideal gas: no pending update; it leaves the face weights and the
+// reciprocal of the preconditioner's diagonal for the passes that follow.
+template <class TS>
+__device__ __forceinline__ bool pass_first_staged(const PressureRow<double, false>& op, const Work<TS>& g,
+                                                  const NewtonArgs& na, Smem<PressureRow<double, false>>& sm, Sync& y,
+                                                  const double* pc, double* pn, double Mbig, double* idg, bool raw) {
+  using Op = PressureRow<double, false>;
+  constexpr int C = Op::C, kStage = 4, kRow = 4 * C * 32;  // a slot: p, h, eta, b
+  const DevParams& P = op.P;
+  Shared& S = sm.S;
+  const int lane = threadIdx.x & 31;
+  double* const stage = reinterpret_cast<double*>(sm.ring[threadIdx.x >> 5]) + lane;
+  acc_clear(S);
+  NewtonSums sum;
+  for_tasks<Op::W>(g, [&](int task) {
+    Op::State st{};
+    double bl[C];
+    int ol[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      bl[c] = 0.0;
+      ol[c] = 0;
+    }
+    auto copy = [&](int it, int c, int n) {
+      double* d = stage + (it & (kStage - 1)) * kRow + c * 32;
+      copy_async(d, pc + n);
+      copy_async(d + C * 32, op.hh + n);
+      copy_async(d + 2 * C * 32, op.eta + n);
+      copy_async(d + 3 * C * 32, na.b + n);
+    };
+    const StagedRows<C, kStage> R(g.G, task);
+    R.start(copy);
+#pragma unroll 1
+    for (int it = 0; it < R.count(); ++it) {
+      int on[C];
+      R.wait(it, on);
+      double w[1][C], bn[C], out[1][C], wc[1][C];
+      Op::Row n;
+      Op::Emit em;
+      const double* d = stage + (it & (kStage - 1)) * kRow;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        w[0][c] = d[c * 32];
+        n.h[c] = d[(C + c) * 32];
+        n.e[c] = d[(2 * C + c) * 32];
+        bn[c] = d[(3 * C + c) * 32];
+        em.vd[c] = 0.0;  // V_mod takes the diagonal's place
+      }
+      R.next(it, copy);
+      op.step(st, w, n, em, out, wc);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        if (it >= 2 && R.own[c]) {
+          const int o = ol[c];
+          const double pv = wc[0][c];
+          const bool fl = P.floor_on && !(pv >= P.p_floor);
+          const double vs = fl ? Mbig : op.a, V = fl ? floored_V(op, Mbig, pv) : op.a * pv;
+          const double gv = out[0][c] + V - bl[c], id = 1.0 / (vs + em.dg[c]);
+          const double r0 = raw ? -gv * id : (double)(TS)(-gv * id);
+          pn[o] = pv;
+          if (!raw) {  // GMRES reads the right-hand side again at a restart, and the slopes
+            na.g[o] = -gv;
+            na.vdiag[o] = vs;
+          }
+          idg[o] = id;
+          op.kx[o] = em.kx[c];
+          op.ky[o] = em.ky[c];
+          g.V0n[o] = (TS)(raw ? -gv : r0);
+          sum.add(P, gv, r0, pv);
+        }
+        bl[c] = bn[c];
+        ol[c] = on[c];
+      }
+    }
+  });
+  count(g, S, 1, Op::kCoef + 6 + (raw ? 0 : 2));
+  return sum.template end<Op::W>(S, y);
+}
+// The rows come through slots two ahead, with the vectors of the pending update; at most
+// kMaxPending of them fit.
+constexpr int kMaxPending = 8;
+template <class TS>
+__device__ __forceinline__ bool pass_faces_staged(const PressureRow<double, false>& op, const Work<TS>& g,
+                                                  const NewtonArgs& na, Smem<FaceRow<double>>& sm, Sync& y,
+                                                  const double* pc, double* pn, double Mbig, const double* id,
+                                                  double* idn, bool pending, bool dp_live) {
+  using Op = FaceRow<double>;
+  constexpr int C = Op::C, kStage = 3, kRow = (6 + kMaxPending) * C * 32;
+  static_assert(kStage * kRow * 8 <= Ring<Op, double>::kBytes, "the stages live in the ring");
+  const DevParams& P = op.P;
+  Shared& S = sm.S;
+  const int lane = threadIdx.x & 31, nv = pending ? S.nalpha : 0;
+  double* const stage = reinterpret_cast<double*>(sm.ring[threadIdx.x >> 5]);
+  acc_clear(S);
+  NewtonSums sum;
+  Op f{};
+  const double zero[C] = {};
+  for_tasks<Op::W>(g, [&](int task) {
+    Op::State st{};
+    double bl[C], il[C];
+    int ol[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      bl[c] = il[c] = 0.0;
+      ol[c] = 0;
+    }
+    // a slot: p, b, kx, ky, id, the part of the update that is formed already, then the vectors
+    int sc = 0, sr = 0;  // slots of the copies and of the row in work
+    auto copy = [&](int, int c, int n) {
+      double* d = stage + sc * kRow + lane + c * 32;
+      copy_async(d, pc + n);
+      copy_async(d + C * 32, na.b + n);
+      copy_async(d + 2 * C * 32, op.kx + n);
+      copy_async(d + 3 * C * 32, op.ky + n);
+      copy_async(d + 4 * C * 32, id + n);
+      if (dp_live) copy_async(d + 5 * C * 32, na.dp + n);
+      TS* t = reinterpret_cast<TS*>(stage + sc * kRow + 6 * C * 32) + lane + c * 32;
+      const TS* v = g.V + n + g.G.N;
+      if (nv > 0) copy_async(t, g.V0 + n);
+      for (int i = 1; i < nv; ++i, v += g.G.N) copy_async(t + i * C * 32, v);
+      if (c == C - 1) sc = sc == kStage - 1 ? 0 : sc + 1;
+    };
+    const StagedRows<C, kStage> R(g.G, task);
+    R.start(copy);
+#pragma unroll 1
+    for (int it = 0; it < R.count(); ++it) {
+      int on[C];
+      R.wait(it, on);
+      double w[C], bn[C], in[C], out[C], wc[C];
+      Op::Row n;
+      const double* d = stage + sr * kRow + lane;
+      const TS* t = reinterpret_cast<const TS*>(stage + sr * kRow + 6 * C * 32) + lane;
+      sr = sr == kStage - 1 ? 0 : sr + 1;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        bn[c] = d[(C + c) * 32];
+        n.kx[c] = d[(2 * C + c) * 32];
+        n.ky[c] = d[(3 * C + c) * 32];
+        in[c] = d[(4 * C + c) * 32];
+        double v = 0.0;
+#pragma unroll
+        for (int i = 0; i < kMaxPending; ++i)
+          if (i < nv) v = fma(S.coef[i], (double)t[(i * C + c) * 32], v);
+        w[c] = d[c * 32] + fma(in[c], v, dp_live ? d[(5 * C + c) * 32] : 0.0);
+        wc[c] = st.x[c];
+      }
+      R.next(it, copy);
+      f.complete(st, w, n, zero, out);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        if (it >= 2 && R.own[c]) {
+          const int o = ol[c];
+          const double pv = wc[c];
+          const bool fl = P.floor_on && !(pv >= P.p_floor);
+          const double gv = out[c] + (fl ? floored_V(op, Mbig, pv) : op.a * pv) - bl[c];
+          const double ic = fl ? 1.0 / (Mbig + (1.0 / il[c] - op.a)) : il[c];
+          pn[o] = pv;
+          idn[o] = ic;
+          g.V0n[o] = (TS)-gv;
+          sum.add(P, gv, -gv * ic, pv);
+        }
+        bl[c] = bn[c];
+        il[c] = in[c];
+        ol[c] = on[c];
+      }
+    }
+  });
+  count(g, S, 1 + nv, 7 + (dp_live ? 1 : 0));
+  return sum.template end<Op::W>(S, y);
+}
+template <class TS, bool kRK, bool kLong>
 __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<TS> g, const NewtonArgs& na,
                       Smem<PressureRow<double, kRK>>& smd, Sync& y) {
   using L = PressureRow<double, kRK>;
@@ -1433,10 +1661,18 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   for (it = 0; it < P.Pnewton_max; ++it) {
     const double* scale = scaled ? id : nullptr;
     bool ok = false;
-    if (it == 0) ok = pass_newton<true>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, pending, dp_live, cg);
-    else if (faces) {
-      if constexpr (!kRK) ok = pass_newton_faces(op, g, na, sm_faces, y, pc, pn, Mbig, scale, id, idn, pending, dp_live);
-    } else ok = pass_newton<false>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, pending, dp_live, cg);
+    if constexpr (kRK) {
+      ok = it == 0 ? pass_newton<true>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, false, false, cg)
+                   : pass_newton<false>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, pending, dp_live, cg);
+    } else if (it == 0) {
+      if constexpr (kLong) ok = pass_first_staged(op, g, na, smd, y, pc, pn, Mbig, idn, cg);
+      else ok = pass_newton<true>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, false, false, cg);
+    } else if (faces && (!kLong || (scaled && (!pending || S.nalpha <= kMaxPending)))) {
+      if constexpr (kLong) ok = pass_faces_staged(op, g, na, sm_faces, y, pc, pn, Mbig, id, idn, pending, dp_live);
+      else ok = pass_newton_faces(op, g, na, sm_faces, y, pc, pn, Mbig, scale, id, idn, pending, dp_live);
+    } else {
+      ok = pass_newton<false>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, pending, dp_live, cg);
+    }
     if (!ok) return GM_SYNC;
     {
       double* q = id;
@@ -1569,7 +1805,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   }
   return worst;
 }
-template <class TS, bool kRK>
+template <bool kLong, class TS, bool kRK>
 __device__ __forceinline__ void newton_body(const NewtonJob<TS, kRK>& j) {
   using Op = PressureRow<double, kRK>;
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -1578,20 +1814,20 @@ __device__ __forceinline__ void newton_body(const NewtonJob<TS, kRK>& j) {
   if (!kRK) op.P.eos_type = IMEX_IDEAL_GAS;
   op.bind();
   Sync y = sync_begin(j.g, sm.S);
-  const int code = newton<TS, kRK>(op, j.g, j.na, sm, y);
+  const int code = newton<TS, kRK, kLong>(op, j.g, j.na, sm, y);
   record_status(j.g, code);
   solve_end(j.g, sm.S, y, code != GM_SYNC);
 }
-template <class TS, bool kRK>
+template <class TS, bool kRK, bool kLong>
 __global__ void __launch_bounds__(32 * PressureRow<double, kRK>::W, 1)
     k_newton(const __grid_constant__ NewtonJob<TS, kRK> j) {
-  newton_body(j);
+  newton_body<kLong>(j);
 }
 template <class TS, bool kRK>
 __global__ void __launch_bounds__(32 * PressureRow<double, kRK>::W, 1)
     k_newton_jobs(const NewtonJob<TS, kRK>* jobs, const int* map) {
   __shared__ JobCopy<NewtonJob<TS, kRK>> s;
-  newton_body(copy_job(s, jobs + map[blockIdx.x]));
+  newton_body<false>(copy_job(s, jobs + map[blockIdx.x]));
 }
 
 // ------------------------------------------------------------------ host side
@@ -1787,16 +2023,23 @@ NewtonJob<TS, kRK> newton_job(imex_ctx* ctx, const Cut& k, double* p, const doub
   j.na.bkeys = keys ? ctx->sc->bkey[keys - 1] : nullptr;
   return j;
 }
+// rows per task from which the residual passes copy their rows ahead (pass_first_staged)
+constexpr int kLongRows = 8;
 template <class TS, bool kRK>
 imex_status newton_one(imex_ctx* ctx, double* p, const double* b, int keys) {
   using Op = PressureRow<double, kRK>;
   const size_t smem = sizeof(Smem<Op>);
-  const int cap = capacity<Op>(ctx, k_newton<TS, kRK>, smem);
+  const int cap = capacity<Op>(ctx, k_newton<TS, kRK, false>, smem);
   if (cap < 1) return set_error(ctx, IMEX_ERR_CUDA, "solver kernel does not fit on an SM");
   const Cut k = make_cut<Op>(ctx, cap);
   const NewtonJob<TS, kRK> j = newton_job<TS, kRK>(ctx, k, p, b, keys);
   prof_begin(ctx);
-  const imex_status s = launch_one<Op>(ctx, k_newton<TS, kRK>, j, k.nblk, smem);
+  imex_status s;
+  // both instances have one block per SM, so the cut fits either
+  if (!kRK && k.G.L >= kLongRows && capacity<Op>(ctx, k_newton<TS, kRK, !kRK>, smem) >= k.nblk)
+    s = launch_one<Op>(ctx, k_newton<TS, kRK, !kRK>, j, k.nblk, smem);
+  else
+    s = launch_one<Op>(ctx, k_newton<TS, kRK, false>, j, k.nblk, smem);
   prof_end(ctx, F_NEWTON, 0.0, 1);
   return s;
 }

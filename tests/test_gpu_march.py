@@ -95,6 +95,32 @@ def test_march_newton_matches_the_tile_kernels(nx, ny, eos, precision):
     assert rel(res[1], res[0]) <= 1e-9, (n, rel(res[1], res[0]))
 
 
+@pytest.mark.parametrize("nx,ny,kind", [(1201, 601, "vortex"), (700, 1100, "blast")])
+@pytest.mark.parametrize("floors", [False, True])
+@pytest.mark.parametrize("precision,restart", [("fp64", 30), ("fp64", 12), ("fp64", 3), ("mixed", 30)])
+def test_march_newton_of_long_tasks(nx, ny, kind, floors, precision, restart):
+    """Tasks of eight rows and more (some short at the last row), whose residual passes copy their
+    rows ahead: with few and many vectors in the pending update, with cells floored after the
+    first iterate.  Tolerance as above."""
+    res = []
+    prob = {"vortex": vortex, "blast": open_blast}[kind](nx, ny)
+    for arith in ("exact", "fast"):
+        sv = ix.Solver.for_problem(prob, 2, dict(B_FORM, arith=arith, p_floor=0.05, theta=0.5, precision=precision,
+                                                 gmres_restart=restart))
+        for name in ("Qe", "Qs"):
+            sv.set_buffer(name, sv.cons())
+        sv.set_scalars(vx_max=0.8, vy_max=0.9)
+        sv.prepare_operator("pressure_L", 2.0 * min(prob.dx, prob.dy))
+        b = 1.5 + 0.3 * np.sin(0.05 * np.arange(sv.N))
+        if floors:
+            b[::11] = 0.02
+        p, st = sv.nested_newton(np.full(sv.N, 0.9), b)
+        assert st["newton_iters"] >= 1
+        res.append(p)
+        sv.close()
+    assert rel(res[1], res[0]) <= 1e-9, rel(res[1], res[0])
+
+
 def test_march_falls_back_where_conjugate_gradients_break_down():
     """A negative face weight (an operator that is not positive definite) hands the solve to GMRES."""
     sv, prob = _solver("vortex", 63, 41, B_FORM)
