@@ -389,6 +389,74 @@ struct k_reconstruct_var {
   }
 };
 
+// The same for large grids: a thread marches `rows` rows up one column.  The five values of its
+// column stay in registers, so a row costs one value of a new line and four of lines that the
+// caches hold, and the column maps are formed once; the values of the next row are asked for
+// before the current row's arithmetic.  What bounds it is the instruction stream: the fast WENO5
+// issues 117 FP64 and 120 other instructions per value and keeps the FP64 pipe 56 % busy (16
+// warps per SM at 92 registers; fewer registers spill and cost more), 3.5 TB/s on 2048^2.
+template <bool kOpen, bool kFast>
+struct k_reconstruct_rows {
+  IMEX_BOUNDS(kThreads, 0)
+  static __device__ __forceinline__ void run(IMEX_BLK, DevParams Pin, const double* __restrict__ Q,
+                                                                 double* __restrict__ w, int rows) {
+    const DevParams P = bc_params<kOpen>(Pin);
+    const long long N = P.N;
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    int i, run;
+    cell_of(P, t, i, run);
+    const int j0 = run * rows;
+    if (j0 >= P.ny) return;
+    const int j1 = P.ny - j0 < rows ? P.ny : j0 + rows;
+    const int k = blockIdx.y;
+    const bool vortex = P.recon == IMEX_Minmod && P.vortex_minmod;
+    const double* a = Q + k * N;
+    double* o = w + k * N + i + (long long)P.nx * j0;
+    const int im2 = cix(P, i - 2), im1 = cix(P, i - 1), ip1 = cix(P, i + 1), ip2 = cix(P, i + 2);
+    double v[5], u[5];  // the stencils along x and y
+    {
+      const double* r = a + (long long)P.nx * j0;
+      v[0] = __ldg(r + im2);
+      v[1] = __ldg(r + im1);
+      v[3] = __ldg(r + ip1);
+      v[4] = __ldg(r + ip2);
+  #pragma unroll
+      for (int d = 0; d < 5; ++d) u[d] = __ldg(a + (long long)P.nx * cjy(P, j0 + d - 2) + i);
+    }
+  #pragma unroll 1
+    for (int j = j0; j < j1; ++j, o += P.nx) {
+      double nv[4] = {0.0, 0.0, 0.0, 0.0}, nu = 0.0;
+      if (j + 1 < j1) {
+        const double* r = a + (long long)P.nx * (j + 1);
+        nu = __ldg(a + (long long)P.nx * cjy(P, j + 3) + i);
+        nv[0] = __ldg(r + im2);
+        nv[1] = __ldg(r + im1);
+        nv[2] = __ldg(r + ip1);
+        nv[3] = __ldg(r + ip2);
+      }
+      v[2] = u[2];
+      double xl, xr, yl, yr;
+      if (kFast && P.recon == IMEX_WENO5) {
+        weno5_fast_xy(v, u, xl, xr, yl, yr);
+      } else {
+        recon_1d<kFast>(P.recon, v[0], v[1], v[2], v[3], v[4], xl, xr, false);
+        recon_1d<kFast>(P.recon, u[0], u[1], u[2], u[3], u[4], yl, yr, vortex);
+      }
+      o[0] = xl;
+      o[8 * N] = xr;
+      o[16 * N] = yl;
+      o[24 * N] = yr;
+  #pragma unroll
+      for (int d = 0; d < 4; ++d) u[d] = u[d + 1];
+      u[4] = nu;
+      v[0] = nv[0];
+      v[1] = nv[1];
+      v[3] = nv[2];
+      v[4] = nv[3];
+    }
+  }
+};
+
 // ---------------------------------------------------------------- flux updates
 // RusanovC_Update (flux.cpp:409-455) or Pressure_flux_Update (flux.cpp:290-326) with the
 // B slots of the face states taken from cell B of u_con (main.cpp:447-467).
@@ -1130,6 +1198,22 @@ imex_status launch_stage_combine(imex_ctx* ctx, int rks) {
   return IMEX_OK;
 }
 
+// The ConsState reconstruction of nvar variables: by rows where the grid fills every SM's 2048
+// threads with two rows a thread (up to 16), else one thread per value, which has the shorter
+// chain.  Measured, us: 700 x 450 29 -> 25, 768^2 37 -> 35, 1024^2 72 -> 68, 2048^2 268 -> 241;
+// with one row a thread 115 at 1024^2 and 11 against 9 on 251 x 173.
+static void reconstruct_var(imex_ctx* ctx, const double* Q, int nvar) {
+  const DevParams& P = ctx->P;
+  const long long fit = (long long)P.N * nvar / ((long long)ctx->num_sms * 2048);
+  if (fit < 2) {
+    IMEX_LAUNCH_BC_ARITH(P, k_reconstruct_var, (dim3(blocks_for(P.N), nvar)), kThreads, 0, ctx->stream, P, Q, ctx->w);
+    return;
+  }
+  const int rows = fit < 16 ? (int)fit : 16;
+  const long long threads = (long long)P.nx * ((P.ny + rows - 1) / rows);
+  IMEX_LAUNCH_BC_ARITH(P, k_reconstruct_rows, (dim3(blocks_for(threads), nvar)), kThreads, 0, ctx->stream, P, Q, ctx->w,
+                       rows);
+}
 // full = true stores all 8 variables (the public buffer); the stage needs only 0..4
 imex_status launch_reconstruct(imex_ctx* ctx, bool full) {
   const int nstore = full ? 8 : 5;
@@ -1139,8 +1223,7 @@ imex_status launch_reconstruct(imex_ctx* ctx, bool full) {
     IMEX_LAUNCH_BC_ARITH(ctx->P, k_reconstruct_prim, blocks_for(ctx->P.N), kThreads, 0, ctx->stream, ctx->P, ctx->Qe,
                          ctx->w, nstore);
   else
-    IMEX_LAUNCH_BC_ARITH(ctx->P, k_reconstruct_var, (dim3(blocks_for(ctx->P.N), nstore)), kThreads, 0, ctx->stream,
-                         ctx->P, ctx->Qe, ctx->w);
+    reconstruct_var(ctx, ctx->Qe, nstore);
   LAUNCH_CHECK(ctx, "k_reconstruct");
   prof_end(ctx, F_RECON, BYTES(nread + 4 * nstore), 1);
   return IMEX_OK;
@@ -1177,7 +1260,7 @@ imex_status launch_ct(imex_ctx* ctx, int variant) {
     LAUNCH_CHECK(ctx, "k_ct_corner");
   } else if (variant == 2) {
     if (P.reconstate == IMEX_PrimState) IMEX_LAUNCH_BC_ARITH(P, k_reconstruct_prim, nb, kThreads, 0, s, P, ctx->cons, ctx->w, 8);
-    else IMEX_LAUNCH_BC_ARITH(P, k_reconstruct_var, (dim3(nb, 8)), kThreads, 0, s, P, ctx->cons, ctx->w);
+    else reconstruct_var(ctx, ctx->cons, 8);
     LAUNCH_CHECK(ctx, "k_reconstruct(u_con)");
     launch<k_ct_legacy_faces>(ctx, nb, kThreads, 0, s, P, ctx->w, ctx->chit, ctx->Et);
     LAUNCH_CHECK(ctx, "k_ct_legacy_faces");
@@ -1258,7 +1341,7 @@ imex_status launch_ct_diag(imex_ctx* ctx, double* out16) {
   cudaStream_t s = ctx->stream;
   double *cp0 = ctx->chit, *c0p = ctx->Et, *rp0 = ctx->Epp, *r0p = ctx->vscale;
   if (P.reconstate == IMEX_PrimState) IMEX_LAUNCH_BC_ARITH(P, k_reconstruct_prim, nb, kThreads, 0, s, P, ctx->cons, ctx->w, 8);
-  else IMEX_LAUNCH_BC_ARITH(P, k_reconstruct_var, (dim3(nb, 8)), kThreads, 0, s, P, ctx->cons, ctx->w);
+  else reconstruct_var(ctx, ctx->cons, 8);
   k_ct_diag_faces<<<nb, kThreads, 0, s>>>(P, ctx->w, cp0, c0p, rp0, r0p);
   int nred = nb < ctx->max_blocks ? nb : ctx->max_blocks;
   k_ct_diag_stats<<<nred, kThreads, 0, s>>>(P, cp0, c0p, rp0, r0p, ctx->cons, ctx->partial);
