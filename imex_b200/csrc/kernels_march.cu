@@ -6,6 +6,14 @@
 namespace imex {
 namespace march {
 
+// The B form's operator in the mixed form: its FP32 rows need half the registers and half the ring,
+// which leaves room for twelve warps instead of eight (the FP64 refinement passes, a few per solve,
+// spill 260 bytes), and its ring of twelve vectors makes loads ahead past it cost more registers than
+// they hide.  A pass waits on its own chain of loads and arithmetic, so warps count.  Whole step of
+// the 1024^2 random field, us, by warps / FP64 vectors in the ring / loaded ahead: 8/8/5 7870, 12/5/5
+// 7702, 12/5/0 7423, 12/6/0 7287, 12/7/0 7819 (too little L1 left), 16/4/0 7580, 10/6/5 8244.
+// The FP64 solve keeps eight warps: it needs their 255 registers.
+using MagBMixed = MagBRow<double, 12, 6, 0>;
 // The solves that run here: the fast arithmetic (the exact one keeps the reference's operation
 // order, which the face forms do not), global dissipation (the energy operator has none) and,
 // in the A form, periodic boundaries (an open tile extrapolates A past the edge).  The other
@@ -26,7 +34,7 @@ imex_status gmres_solve(imex_ctx* ctx, int op, int fam, double* x, const double*
   }
   if (op == IMEX_OP_ENERGY) return solve<EnergyRow<double>>(ctx, false, fam, IMEX_MIXED_PRESSURE, x, b, scratch);
   if (op == IMEX_OP_MAGNETIC_B)
-    return solve<MagBRow<double>>(ctx, false, fam, IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B, x, b, scratch);
+    return solve<MagBRow<double>, MagBMixed>(ctx, false, fam, IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B, x, b, scratch);
   return solve<MagARow<double>>(ctx, false, fam, IMEX_MIXED_MAGNETIC, x, b, scratch);
 }
 imex_status newton_solve(imex_ctx* ctx, double* p, const double* b, int keys) {
@@ -39,7 +47,7 @@ imex_status batch_build(BatchSolvePlan* plan, const std::vector<imex_ctx*>& memb
   if (op == IMEX_OP_MAGNETIC_A)
     return add_solves<MagARow<double>>(plan, members, IMEX_MIXED_MAGNETIC, F_GMRES_MAG_A, magnetic_system);
   if (op == IMEX_OP_MAGNETIC_B)
-    return add_solves<MagBRow<double>>(plan, members, IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B, F_GMRES_MAG_B,
+    return add_solves<MagBRow<double>, MagBMixed>(plan, members, IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B, F_GMRES_MAG_B,
                                        magnetic_system);
   if (op == IMEX_OP_ENERGY)
     return add_solves<EnergyRow<double>>(plan, members, IMEX_MIXED_PRESSURE, F_GMRES_ENERGY, energy_system);

@@ -415,14 +415,15 @@ struct MagBCoef {
     cy = sc->B_max_y * P.dy / (P.dy * P.dy);
   }
 };
-template <class T_>
+// W_, R_, A_: warps per block, vectors in the ring, vectors past it loaded ahead.
+template <class T_, int W_ = 8, int R_ = 8, int A_ = 5>
 struct MagBRow : MagBCoef {
   using T = T_;
-  static constexpr int M = 3, H = 1, C = 1, kLag = 0, W = 8, R = 8, kDots = 8, kAhead = 5;
+  static constexpr int M = 3, H = 1, C = 1, kLag = 0, W = W_, R = R_, kDots = 8, kAhead = A_;
   static constexpr int kCoef = 4;
   template <class U>
-  __device__ __forceinline__ MagBRow<U> as() const {
-    MagBRow<U> o;
+  __device__ __forceinline__ MagBRow<U, W_, R_, A_> as() const {
+    MagBRow<U, W_, R_, A_> o;
     static_cast<MagBCoef&>(o) = *this;
     return o;
   }

@@ -1960,18 +1960,18 @@ imex_status launch_one(imex_ctx* ctx, K kernel, const Job& job, int nblk, size_t
                     "cooperative launch");
 }
 
-template <class Op>
+// Op: the FP64 solve's operator; MOp: the mixed form's
+template <class Op, class MOp = Op>
 imex_status solve(imex_ctx* ctx, bool jac, int fam, int kind, double* x, const double* b, const Scratch* scratch) {
-  const size_t smem = sizeof(Smem<Op>);
-  const Op op = make_op<Op>(ctx, jac);
   prof_begin(ctx);
   imex_status s;
   if (scratch || !is_mixed(ctx, kind)) {
+    const size_t smem = sizeof(Smem<Op>);
     GmresJob<Op> j{};
     const int cap = capacity<Op>(ctx, k_gmres<Op>, smem);
     if (cap < 1) return set_error(ctx, IMEX_ERR_CUDA, "solver kernel does not fit on an SM");
     const Cut k = make_cut<Op>(ctx, cap);
-    j.op = op;
+    j.op = make_op<Op>(ctx, jac);
     j.g = make_work<double>(ctx, k, Op::M, fam);
     if (scratch) {
       j.g.V = j.g.V0 = scratch->V;
@@ -1983,12 +1983,13 @@ imex_status solve(imex_ctx* ctx, bool jac, int fam, int kind, double* x, const d
     j.b = b;
     s = launch_one<Op>(ctx, k_gmres<Op>, j, k.nblk, smem);
   } else {
-    MixedJob<Op> j{};
-    const int cap = capacity<Op>(ctx, k_mixed<Op>, smem);
+    const size_t smem = sizeof(Smem<MOp>);
+    MixedJob<MOp> j{};
+    const int cap = capacity<MOp>(ctx, k_mixed<MOp>, smem);
     if (cap < 1) return set_error(ctx, IMEX_ERR_CUDA, "solver kernel does not fit on an SM");
-    const Cut k = make_cut<Op>(ctx, cap);
-    j.op = op;
-    j.g = make_work<float>(ctx, k, Op::M, fam);
+    const Cut k = make_cut<MOp>(ctx, cap);
+    j.op = make_op<MOp>(ctx, jac);
+    j.g = make_work<float>(ctx, k, MOp::M, fam);
     j.g.tol_abs = 0.0;
     j.g.max_restarts = 1;
     j.x = x;
@@ -1996,7 +1997,7 @@ imex_status solve(imex_ctx* ctx, bool jac, int fam, int kind, double* x, const d
     j.b = b;
     j.max_sweeps = ctx->cfg.mixed_max_refine;
     j.tol = outer_tol(ctx);
-    s = launch_one<Op>(ctx, k_mixed<Op>, j, k.nblk, smem);
+    s = launch_one<MOp>(ctx, k_mixed<MOp>, j, k.nblk, smem);
   }
   prof_end(ctx, fam, 0.0, 1);
   return s;
@@ -2105,21 +2106,20 @@ imex_status add_chunks(BatchSolvePlan* plan, const std::vector<imex_ctx*>& membe
   }
   return IMEX_OK;
 }
-template <class Op, class Sys>
+template <class Op, class MOp = Op, class Sys>
 imex_status add_solves(BatchSolvePlan* plan, const std::vector<imex_ctx*>& members, int kind, int fam, Sys system) {
-  const size_t smem = sizeof(Smem<Op>);
   if (!is_mixed(members[0], kind))
-    return add_chunks<Op, GmresJob<Op>>(plan, members, k_gmres_jobs<Op>, smem, [&](imex_ctx* m, const Cut& k) {
+    return add_chunks<Op, GmresJob<Op>>(plan, members, k_gmres_jobs<Op>, sizeof(Smem<Op>), [&](imex_ctx* m, const Cut& k) {
       GmresJob<Op> j{};
       j.op = make_op<Op>(m);
       j.g = make_work<double>(m, k, Op::M, fam);
       system(m, &j.x, &j.b);
       return j;
     });
-  return add_chunks<Op, MixedJob<Op>>(plan, members, k_mixed_jobs<Op>, smem, [&](imex_ctx* m, const Cut& k) {
-    MixedJob<Op> j{};
-    j.op = make_op<Op>(m);
-    j.g = make_work<float>(m, k, Op::M, fam);
+  return add_chunks<MOp, MixedJob<MOp>>(plan, members, k_mixed_jobs<MOp>, sizeof(Smem<MOp>), [&](imex_ctx* m, const Cut& k) {
+    MixedJob<MOp> j{};
+    j.op = make_op<MOp>(m);
+    j.g = make_work<float>(m, k, MOp::M, fam);
     j.g.tol_abs = 0.0;
     j.g.max_restarts = 1;
     system(m, &j.x, &j.b);
