@@ -194,6 +194,8 @@ _SIGS = {
     "imex_kernel_launch_count": (C.c_int, [C.c_void_p, C.POINTER(C.c_longlong)]),
     "imex_set_barrier_timeout": (C.c_int, [C.c_void_p, C.c_double]),
     "imex_selftest_barrier": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_double, _D]),
+    "imex_selftest_pass_end": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_double, C.c_double, _D,
+                                         C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "imex_selftest_fp64": (C.c_int, [C.c_void_p, _D, _D]),
 }
 
@@ -388,6 +390,14 @@ class Solver:
         self._check(self.lib.imex_selftest_barrier(self.ctx, iterations, phantom_blocks, timeout_s,
                                                    C.byref(us)))
         return us.value
+
+    def selftest_pass_end(self, iterations: int, phantom_blocks: int = 0, late_s: float = 0.0,
+                          timeout_s: float = 1.0) -> dict:
+        """Pass ends of the row-marching solves: status, mean microseconds, blocks that gave up, blocks."""
+        us, out, blocks = C.c_double(), C.c_int(), C.c_int()
+        rc = self.lib.imex_selftest_pass_end(self.ctx, iterations, phantom_blocks, late_s, timeout_s, C.byref(us),
+                                             C.byref(out), C.byref(blocks))
+        return {"status": rc, "us": us.value, "gave_up": out.value, "blocks": blocks.value}
 
     def kernel_launches(self) -> int:
         n = C.c_longlong()

@@ -926,6 +926,14 @@ imex_status imex_selftest_barrier(imex_ctx* ctx, int iterations, int phantom_blo
   imex_status s = run_barrier_selftest(ctx, iterations, phantom_blocks, timeout_s, us_per_barrier);
   return s != IMEX_OK ? s : device_status(ctx);
 }
+imex_status imex_selftest_pass_end(imex_ctx* ctx, int iterations, int phantom_blocks, double late_s, double timeout_s,
+                                   double* us_per_pass_end, int* gave_up, int* blocks) {
+  if (!ctx || iterations < 0 || phantom_blocks < 0 || !(timeout_s > 0.0) || timeout_s > 60.0) return IMEX_ERR_INVALID;
+  if (!(late_s >= 0.0) || late_s > 1.0) return IMEX_ERR_INVALID;
+  imex_status s =
+      run_pass_end_selftest(ctx, iterations, phantom_blocks, late_s, timeout_s, us_per_pass_end, gave_up, blocks);
+  return s != IMEX_OK ? s : device_status(ctx);
+}
 imex_status imex_selftest_fp64(imex_ctx* ctx, double* dfma_per_s, double* ddiv_per_s) {
   if (!ctx) return IMEX_ERR_INVALID;
   return run_fp64_selftest(ctx, dfma_per_s, ddiv_per_s);

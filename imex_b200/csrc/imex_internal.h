@@ -99,9 +99,9 @@ struct SyncState {
   int abort;
   int pad1;
   long long wait_cycles;  // bound of any single barrier wait, in SM clock cycles
-  // pass ends of the row-marching kernels (march.cuh): arrivals so far, over all launches; their
-  // number when the next launch starts; the mark of a launch that gave up, if any
-  unsigned long long arrivals, epoch, abort_at;
+  // pass ends of the row-marching kernels (march.cuh): arrivals so far, over all launches (the top
+  // bit: a launch gave up); their number when the next launch starts
+  unsigned long long arrivals, epoch;
 };
 
 }  // namespace imex
@@ -248,6 +248,8 @@ imex_status run_gmres(imex_ctx* ctx, int op, double* x, const double* b);
 imex_status run_nested_newton(imex_ctx* ctx, double* p, const double* b);
 imex_status set_newton_state(imex_ctx* ctx, const double* pf, double mbig);
 imex_status run_fp64_selftest(imex_ctx* ctx, double* dfma_per_s, double* ddiv_per_s);
+imex_status run_pass_end_selftest(imex_ctx* ctx, int iterations, int phantom_blocks, double late_s, double timeout_s,
+                                  double* us, int* gave_up, int* blocks);
 imex_status run_barrier_selftest(imex_ctx* ctx, int iterations, int phantom_blocks, double timeout_s,
                                  double* us_per_barrier);
 

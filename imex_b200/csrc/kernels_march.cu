@@ -5,6 +5,38 @@
 
 namespace imex {
 namespace march {
+namespace {
+
+// Every block runs `iters` pass ends over the launched blocks and `phantom` others that were never
+// launched; the first block, whose verdict is the launch's as in a solve, comes `late` cycles after
+// the rest to the last of them.  *gave_up: blocks that did not get through with the right sum.
+constexpr int kSelfWarps = 8;
+__global__ void __launch_bounds__(32 * kSelfWarps, 1)
+    k_pass_end_selftest(SyncState* sync, double* partial, DevStats* st, int phantom, int iters, long long late,
+                        long long limit, long long* cycles, int* gave_up) {
+  __shared__ Shared S;
+  Sync y{sync, ld_relaxed(&sync->epoch), 0ull, limit, (int)gridDim.x + phantom, (int)blockIdx.x, partial};
+  const long long t0 = clock64();
+  bool ok = true;
+  for (int k = 0; ok && k < iters; ++k) {
+    if (blockIdx.x == 0 && k + 1 == iters) {
+      const long long t1 = clock64();
+      while (clock64() - t1 < late) {
+      }
+    }
+    acc_clear(S);
+    if ((threadIdx.x & 31) == 0) S.acc[threadIdx.x >> 5][0] = 1.0;
+    ok = pass_end<kSelfWarps>(y, S, 1) && S.red[0] == (double)(kSelfWarps * y.nblk);
+  }
+  if (threadIdx.x != 0) return;
+  if (!ok) atomicAdd(gave_up, 1);
+  if (blockIdx.x != 0) return;
+  *cycles = clock64() - t0;
+  if (!ok) atomicMax(&st->status, (int)IMEX_ERR_SYNC);
+  else if (y.seq > 0) st_relaxed(&sync->epoch, y.base + y.seq * (unsigned long long)y.nblk);
+}
+
+}  // namespace
 
 // The B form's operator in the mixed form: its FP32 rows need half the registers and half the ring,
 // which leaves room for twelve warps instead of eight (the FP64 refinement passes, a few per solve,
@@ -62,4 +94,36 @@ size_t scratch_partials(imex_ctx* ctx) {
 }
 
 }  // namespace march
+
+imex_status run_pass_end_selftest(imex_ctx* ctx, int iterations, int phantom_blocks, double late_s, double timeout_s,
+                                  double* us, int* gave_up, int* blocks) {
+  const int nb = ctx->num_sms < kMaxBlocks ? ctx->num_sms : kMaxBlocks;
+  if (2LL * (nb + phantom_blocks) * march::kSlots > ctx->partial_len)
+    return set_error(ctx, IMEX_ERR_INVALID, "pass-end self-test: too many phantom blocks");
+  const double khz = ctx->clock_khz > 0 ? (double)ctx->clock_khz : 2.0e6;
+  long long late = (long long)(late_s * khz * 1e3), limit = (long long)(timeout_s * khz * 1e3) + 1;
+  long long* cycles = reinterpret_cast<long long*>(ctx->red);
+  int* count = reinterpret_cast<int*>(ctx->red + 1);
+  cudaError_t e = cudaMemsetAsync(ctx->red, 0, 2 * sizeof(double), ctx->stream);
+  if (e != cudaSuccess) return cuda_check(ctx, e, "pass-end self-test");
+  void* params[] = {(void*)&ctx->sync, (void*)&ctx->partial, (void*)&ctx->st, (void*)&phantom_blocks, (void*)&iterations,
+                    (void*)&late,      (void*)&limit,        (void*)&cycles,  (void*)&count};
+  e = cudaLaunchCooperativeKernel((const void*)march::k_pass_end_selftest, dim3(nb), dim3(32 * march::kSelfWarps), params, 0,
+                                  ctx->stream);
+  if (e != cudaSuccess) return cuda_check(ctx, e, "pass-end self-test launch");
+  ctx->kernel_launches += 1;
+  double h[2] = {0.0, 0.0};
+  e = cudaMemcpyAsync(h, ctx->red, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) return cuda_check(ctx, e, "pass-end self-test");
+  long long spent = 0;
+  int out = 0;
+  std::memcpy(&spent, &h[0], sizeof(spent));
+  std::memcpy(&out, &h[1], sizeof(out));
+  if (us) *us = iterations > 0 ? (double)spent / iterations / (khz * 1e-3) : 0.0;
+  if (gave_up) *gave_up = out;
+  if (blocks) *blocks = nb;
+  return IMEX_OK;
+}
+
 }  // namespace imex

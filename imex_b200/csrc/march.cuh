@@ -703,7 +703,11 @@ __device__ __forceinline__ double warp_min(double x) {
 // array of per-block flags that every block reads takes 11 thousand (148 readers of the same
 // lines hold up the writers), relaxed polls closed by a fence 5.3, cluster leaders with the sums
 // in distributed shared memory 5.0 to 5.3.  The wait is bounded: after `limit` SM cycles the
-// block raises the abort mark and the kernel returns.  The counter grows from launch to launch
+// block gives the launch up, by a compare-and-swap that sets the counter's top bit only while the
+// target is not reached.  The word that counts the arrivals thus also decides: either every block
+// passes this end, or every block leaves here or at a later end, and none takes a launch that
+// others gave up for a whole one.  The bit stays until the host starts the counters again, and
+// launches before that end at their first wait.  The counter grows from launch to launch
 // (SyncState::epoch is its value at the start), so no reset precedes a launch; the first block
 // stores the next epoch when it leaves, which no block reads before the next launch.
 __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
@@ -721,6 +725,17 @@ __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long 
 }
 __device__ __forceinline__ void arrive(unsigned long long* p) {
   asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(p) : "memory");
+}
+constexpr unsigned long long kGaveUp = 1ull << 63;
+// gives the launch up unless the target has been reached in the meantime; the counter as decided
+__device__ __forceinline__ unsigned long long give_up(unsigned long long* p, unsigned long long target) {
+  unsigned long long v = ld_relaxed(p);
+  while (v < target) {
+    const unsigned long long was = atomicCAS(p, v, v | kGaveUp);
+    if (was == v) return v | kGaveUp;
+    v = was;
+  }
+  return ld_acquire(p);
 }
 
 struct Shared {
@@ -772,16 +787,14 @@ __device__ __forceinline__ bool pass_end(Sync& y, Shared& S, int kn, unsigned mi
   }
   int ok = 1;
   if (tid == 0) {
-    const long long t0 = clock64();
-    for (unsigned spin = 0; ok && ld_acquire(&y.s->arrivals) < target; ++spin) {
-      if ((spin & 63u) == 63u) {
-        if (ld_relaxed(&y.s->abort_at) == y.base + 1ull) ok = 0;
-        else if (clock64() - t0 > y.limit) {
-          st_relaxed(&y.s->abort_at, y.base + 1ull);
-          ok = 0;
-        }
-      }
+    unsigned long long v = ld_acquire(&y.s->arrivals);
+    if (v < target) {
+      const long long t0 = clock64();
+      do {
+        v = clock64() - t0 > y.limit ? give_up(&y.s->arrivals, target) : ld_acquire(&y.s->arrivals);
+      } while (v < target);
     }
+    ok = (v & kGaveUp) == 0;
   }
   ok = __syncthreads_and(ok);
   if (!ok) return false;

@@ -440,12 +440,19 @@ imex_status imex_divergence(imex_ctx* ctx, double* face_l2, double* cell_wrapped
  * `seconds` (default 2 s) the waiting CTAs give up, the kernel returns and the
  * call reports IMEX_ERR_SYNC; the context stays usable. */
 imex_status imex_set_barrier_timeout(imex_ctx* ctx, double seconds);
-/* Runs `iterations` device-wide barriers with the solver's CTA count and reports the
- * mean cost per barrier.  `phantom_blocks` > 0 makes the barrier wait for CTAs that
- * were never launched, so the bounded wait must run out after `timeout_s` and the
+/* Runs `iterations` device-wide barriers of the tile kernels (the solves of the exact
+ * arithmetic, the local dissipation and the open A form) with their CTA count and reports
+ * the mean cost per barrier.  `phantom_blocks` > 0 makes the barrier wait for CTAs
+ * that were never launched, so the bounded wait must run out after `timeout_s` and the
  * call must return IMEX_ERR_SYNC (a self-test of the failure path). */
 imex_status imex_selftest_barrier(imex_ctx* ctx, int iterations, int phantom_blocks, double timeout_s,
                                   double* us_per_barrier);
+/* The same for the pass ends of the row-marching solver kernels (all other solves), one block
+ * per SM.  `late_s` <= 1 keeps the first block from the last pass end for that long: with
+ * `timeout_s` below it the others give up, and the launch must end as given up in every block.
+ * *blocks: blocks launched; *gave_up: blocks whose wait was given up (either may be null). */
+imex_status imex_selftest_pass_end(imex_ctx* ctx, int iterations, int phantom_blocks, double late_s, double timeout_s,
+                                   double* us_per_pass_end, int* gave_up, int* blocks);
 /* FP64 throughput of the context's device, measured (no counterpart in the reference):
  * fused multiply-adds per second and IEEE double divisions per second, each from a
  * kernel of independent dependency chains over every SM with no memory traffic.  These

@@ -80,3 +80,21 @@ def test_strong_field_redlich_kwong_is_reported_like_the_reference_fails():
     assert err.value.status in (5, 6, 7, 9)  # Newton cap, non-finite, positivity or EOS iteration cap
     sv.scalars()  # the context still answers after the error
     sv.close()
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 7])
+def test_pass_end_is_given_up_by_every_block_or_by_none(iterations):
+    """The pass end of the row-marching solves, whose last arrival is the first block's, 0.2 s after the
+    others' bound of 0.02 s ran out: that block finds the arrivals complete, and yet the launch counts as
+    given up in every block.  With a bound that is long enough, or without delay, in none."""
+    sv = ix.Solver.for_problem(vortex(64), 2, dict(recon="VanLeer", magfield="StaggerCT"))
+    r = sv.selftest_pass_end(iterations, late_s=0.2, timeout_s=2.0)
+    assert r["status"] == 0 and r["gave_up"] == 0 and r["blocks"] > 1
+    r = sv.selftest_pass_end(iterations, late_s=0.2, timeout_s=0.02)
+    assert r["status"] == 8 and r["gave_up"] == r["blocks"], r
+    r = sv.selftest_pass_end(iterations, phantom_blocks=1, timeout_s=0.02)
+    assert r["status"] == 8 and r["gave_up"] == r["blocks"], r
+    r = sv.selftest_pass_end(200)
+    assert r["status"] == 0 and r["gave_up"] == 0 and 0.0 < r["us"] < 1000.0, r
+    assert sv.step() > 0 and sv.divergence()["face_l2"] < 1e-12
+    sv.close()
