@@ -174,6 +174,11 @@ imex_status write_scalars(imex_ctx* ctx) {
   return cuda_check(ctx, e, "scalar upload");
 }
 
+// The arrival counter of the marching solves from zero: a launch that gave up leaves its mark in it, and
+// every later one ends at its first wait until the mark is gone (march.cuh).  Called wherever a status
+// that may be IMEX_ERR_SYNC is cleared.
+cudaError_t restart_waits(imex_ctx* ctx) { return cudaMemsetAsync(ctx->sync, 0, sizeof(SyncState), ctx->stream); }
+
 // worst status recorded on the device since the last call (resets it)
 // The status of the work queued so far, with one wait: the solve statistics, both EOS
 // flags and (with_scalars) the step scalars come back in one round trip.
@@ -196,8 +201,7 @@ imex_status device_status(imex_ctx* ctx, bool with_scalars = false) {
   if (f2) eos_flag_solve(ctx, &f2, true);
   if (f3) eos_flag_march_clear(ctx);
   if ((f1 || f2 || f3) && s < IMEX_ERR_EOS) s = IMEX_ERR_EOS;
-  // a solve gave up waiting: its arrival counter and epoch no longer agree
-  if (s == IMEX_ERR_SYNC) cudaMemsetAsync(ctx->sync, 0, sizeof(SyncState), ctx->stream);
+  if (s == IMEX_ERR_SYNC) restart_waits(ctx);
   if (s != IMEX_OK) {
     int zero = 0;
     cudaMemcpyAsync(&ctx->st->status, &zero, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
@@ -867,6 +871,7 @@ imex_status imex_reset_stats(imex_ctx* ctx) {
   std::memset(ctx->h_st, 0, sizeof(DevStats));
   ctx->h_st->min_p = 1e300;
   cudaError_t e = cudaMemcpyAsync(ctx->st, ctx->h_st, sizeof(DevStats), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = restart_waits(ctx);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   return cuda_check(ctx, e, "stats reset");
 }

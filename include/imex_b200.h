@@ -438,7 +438,9 @@ imex_status imex_divergence(imex_ctx* ctx, double* face_l2, double* cell_wrapped
 /* Failure detection ---------------------------------------------------------
  * Every device-wide wait inside the persistent solver kernels is bounded: after
  * `seconds` (default 2 s) the waiting CTAs give up, the kernel returns and the
- * call reports IMEX_ERR_SYNC; the context stays usable. */
+ * call reports IMEX_ERR_SYNC; the context stays usable.  An ensemble takes its
+ * members' bounds when it plans its step: at its first step, and at the first one
+ * after imex_batch_configure. */
 imex_status imex_set_barrier_timeout(imex_ctx* ctx, double seconds);
 /* Runs `iterations` device-wide barriers of the tile kernels (the solves of the exact
  * arithmetic, the local dissipation and the open A form) with their CTA count and reports

@@ -98,3 +98,59 @@ def test_pass_end_is_given_up_by_every_block_or_by_none(iterations):
     assert r["status"] == 0 and r["gave_up"] == 0 and 0.0 < r["us"] < 1000.0, r
     assert sv.step() > 0 and sv.divergence()["face_l2"] < 1e-12
     sv.close()
+
+
+VORTEX = dict(recon="VanLeer", magfield="StaggerCT", GMREStol=1e-12)
+AT_ONCE = 1e-9  # a bound of two clock cycles: the first block that has to wait at all gives up
+
+
+def _fresh_run(steps):
+    sv = ix.Solver.for_problem(vortex(64), 2, VORTEX)
+    for _ in range(steps):
+        sv.step()
+    c = sv.cons()
+    sv.close()
+    return c
+
+
+def test_solves_wait_again_after_a_reset_of_the_statistics():
+    """A stage whose solves gave up, and whose status is cleared by imex_reset_stats before a call
+    reads it: the next steps are a fresh context's, bit for bit."""
+    sv = ix.Solver.for_problem(vortex(64), 2, VORTEX)
+    sv.set_barrier_timeout(AT_ONCE)
+    sv.begin_step()
+    sv.stage(0)
+    assert sv.stats()["status"] == 8
+    sv.reset_stats()
+    sv.set_barrier_timeout(2.0)
+    sv.load(vortex(64))
+    sv.step()
+    sv.step()
+    np.testing.assert_array_equal(sv.cons(), _fresh_run(2))
+    sv.close()
+
+
+@pytest.mark.parametrize("streams,graph", [(0, True), (0, False), (2, False)])
+def test_ensemble_waits_again_after_a_wait_ran_out(streams, graph):
+    """The step of an ensemble whose waits run out reports IMEX_ERR_SYNC; with a bound as usual the
+    members' next steps are a fresh ensemble's, bit for bit."""
+    probs = [vortex(64), vortex(48, 96), vortex(80)]
+    batch = ix.Batch(probs, 2, VORTEX, streams=streams, graph=graph)
+    for sv in batch.members:
+        sv.set_barrier_timeout(AT_ONCE)
+    for _ in range(2):
+        with pytest.raises(ix.ImexError) as err:
+            batch.step(1)
+        assert err.value.status == 8
+    for sv in batch.members:
+        sv.set_barrier_timeout(2.0)
+    assert batch.lib.imex_batch_configure(batch.b, streams, 1 if graph else 0) == 0
+    fresh = ix.Batch(probs, 2, VORTEX, streams=streams, graph=graph)
+    for sv, p in zip(batch.members, probs):
+        sv.load(p)
+    batch.step(2)
+    fresh.step(2)
+    for a, b in zip(batch.members, fresh.members):
+        np.testing.assert_array_equal(a.cons(), b.cons())
+    batch.close()
+    fresh.close()
