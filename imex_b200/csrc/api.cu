@@ -200,8 +200,8 @@ imex_status device_status(imex_ctx* ctx, bool with_scalars = false) {
   if (f1) eos_flag_stage(ctx, &f1, true);  // clears it
   if (f2) eos_flag_solve(ctx, &f2, true);
   if (f3) eos_flag_march_clear(ctx);
+  if (s == IMEX_ERR_SYNC) restart_waits(ctx);  // before an EOS flag takes the status's place
   if ((f1 || f2 || f3) && s < IMEX_ERR_EOS) s = IMEX_ERR_EOS;
-  if (s == IMEX_ERR_SYNC) restart_waits(ctx);
   if (s != IMEX_OK) {
     int zero = 0;
     cudaMemcpyAsync(&ctx->st->status, &zero, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);

@@ -154,3 +154,26 @@ def test_ensemble_waits_again_after_a_wait_ran_out(streams, graph):
         np.testing.assert_array_equal(a.cons(), b.cons())
     batch.close()
     fresh.close()
+
+
+def test_solves_wait_again_when_an_eos_flag_hides_the_timed_out_wait():
+    """A status of IMEX_ERR_EOS stands for a timed-out wait too.  The flag is raised by another context's
+    upload (the flags belong to the device): with attraction 1e-300 and pressure 0 the inversion of the
+    Redlich-Kwong EOS starts at T = 1e-300 and triples it each iteration towards 1e-200, past its cap of 200."""
+    rk = ix.Solver.for_problem(vortex(64), 2, dict(VORTEX, eos_type="REDLICH_KWONG", m_alfa=1e-300, m_b=0.1))
+    empty = vortex(64)
+    empty.prim[0], empty.prim[1:8] = 1.0, 0.0
+    sv = ix.Solver.for_problem(vortex(64), 2, VORTEX)
+    sv.set_barrier_timeout(AT_ONCE)
+    rk.load(empty)
+    rk.scalars()  # the upload is done
+    with pytest.raises(ix.ImexError) as err:
+        sv.step()
+    assert err.value.status == 9
+    rk.close()
+    sv.set_barrier_timeout(2.0)
+    sv.load(vortex(64))
+    sv.step()
+    sv.step()
+    np.testing.assert_array_equal(sv.cons(), _fresh_run(2))
+    sv.close()
