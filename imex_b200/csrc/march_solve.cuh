@@ -1655,7 +1655,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   // the other (the slopes of floored cells change between Newton iterations)
   double *id = op.idg, *idn = kRK ? op.idg : na.idg2;
   bool pending = false, dp_live = false, scaled = false;
-  bool cg = !kRK && g.kmax > 1, faces = false;
+  bool cg = !kRK && g.kmax > 1, faces = false, put_slopes = false;
   Smem<FaceRow<double>>& sm_faces = reinterpret_cast<Smem<FaceRow<double>>&>(smd);
   int it, iters = 0, worst = GM_CONVERGED;
   for (it = 0; it < P.Pnewton_max; ++it) {
@@ -1674,6 +1674,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       ok = pass_newton<false>(op, g, na, smd, y, pc, pn, Mbig, scale, idn, pending, dp_live, cg);
     }
     if (!ok) return GM_SYNC;
+    put_slopes = cg;
     {
       double* q = id;
       id = idn;
@@ -1770,12 +1771,19 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   }
   if (lead(g)) g.st->gmres_iters += iters;
   if (it == P.Pnewton_max && lead(g)) atomicMax(&g.st->status, (int)IMEX_NEWTON_MAXIT);
-  // ---- the result in p; floored cells and smallest pressure (implicit_operators.cpp:722-737)
+  // ---- the result in p; floored cells and smallest pressure (implicit_operators.cpp:722-737), and the
+  // slopes of the last residual pass's iterate, which are the J mode's from here on (the reference's
+  // p_freeze), unless that pass wrote them: conjugate gradients do without the plane, so it is written once
+  // a solve instead of once a pass
+  auto put_slope = [&](long long c, double pv) {
+    if (put_slopes) na.vdiag[c] = P.floor_on && !(pv >= P.p_floor) ? Mbig : op.a;
+  };
   if (pending || pc != na.p || P.Pnewton_max <= 0) {
     double nf = 0.0, mn = INFINITY;
     const int na_ = S.nalpha;
     for (long long c = ((long long)blockIdx.x - g.first) * 32 * L::W + threadIdx.x; c < N; c += (long long)g.nblk * 32 * L::W) {
       double pv = pc[c];
+      put_slope(c, pv);
       if (pending) {
         double d = 0.0;
         for (int i = 0; i < na_; ++i) d = fma(S.coef[i], ldv(basis<L>(g, i) + c), d);
@@ -1796,7 +1804,13 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       }
       if (!pass_end<L::W>(y, S, 4, 8u)) return GM_SYNC;
     }
+  } else if (put_slopes) {
+    // without floored cells every slope is the constant a, and the iterate is not read
+    const bool floored = P.floor_on && !(S.red[2] == 0.0 && isfinite(S.red[0]));
+    for (long long c = ((long long)blockIdx.x - g.first) * 32 * L::W + threadIdx.x; c < N; c += (long long)g.nblk * 32 * L::W)
+      put_slope(c, floored ? pc[c] : INFINITY);
   }
+  if (put_slopes) count(g, S, 0, 1);
   if (P.floor_on && lead(g)) {
     const double nf = S.red[2], pmin = S.red[3];
     if ((int)nf > g.st->max_floored) g.st->max_floored = (int)nf;

@@ -166,3 +166,33 @@ def test_march_mixed_magnetic_solve_around_its_ring(nx, ny, kind, restart):
     want, st = sv.gmres("magnetic_B", np.zeros_like(x), b)
     sv.close()
     assert rel(got, want) <= 4 * 6e-8 * 1e3, rel(got, want)
+
+
+def _newton_solver(nx, ny, steps, **settings):
+    prob = vortex(nx, ny)
+    sv = ix.Solver.for_problem(prob, 2, dict(B_FORM, **settings))
+    for name in ("Qe", "Qs"):
+        sv.set_buffer(name, sv.cons())
+    sv.set_scalars(vx_max=0.8, vy_max=0.9)
+    sv.prepare_operator("pressure_L", steps * min(prob.dx, prob.dy))
+    return sv
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("floors", [False, True])
+@pytest.mark.parametrize("nx,ny", [(63, 41), (700, 500)])
+def test_newton_leaves_its_slopes_to_the_jacobian_operator(floors, nx, ny, precision):
+    """IMEX_OP_PRESSURE_J after a nested Newton has the slopes of its last iterate (the reference's p_freeze),
+    whatever was set before.  The operators agree to rounding: 1e-12."""
+    out = []
+    for arith in ("exact", "fast"):
+        sv = _newton_solver(nx, ny, 0.1, arith=arith, p_floor=0.05, theta=0.5, precision=precision)
+        sv.set_newton_state(np.where(np.arange(sv.N) % 3 == 1, -1.0, 1.0), 7.0)
+        b = 1.5 * np.ones(sv.N)
+        if floors:
+            b[::11] = 0.002
+        p, st = sv.nested_newton(np.full(sv.N, 0.9), b)
+        assert st["status"] in (0, 7) and (p < 0.05).any() == floors
+        out.append(sv.apply_operator("pressure_J", _known(sv, "pressure_J")))
+        sv.close()
+    assert rel(out[1], out[0]) <= 1e-12, rel(out[1], out[0])
