@@ -1043,7 +1043,8 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
   double tol_eff = 0.0;
   int iters = 0, code = GM_MAXIT;
   const bool cg = kSym && g.kmax > 1;
-  for (int outer = 0; outer < g.max_restarts; ++outer) {
+  int cycles = g.max_restarts;
+  for (int outer = 0; outer < cycles; ++outer) {
     bool ok = false;
     if constexpr (!kScalar<Op>) {
       ok = pass_residual<false>(op, g, S, y, x, b);
@@ -1068,6 +1069,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
         bool live = true;
         code = cg_solve(kop, g, sm, y, tol_eff, x, live, iters);
         scaled = true;
+        if (code == GM_BREAK) ++cycles;  // GMRES has all of its own
       }
     }
     if (!scaled) {
@@ -1079,7 +1081,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
     if constexpr (kSym) apply_update<Op::M, Op::W>(g, S, x, false, scaled ? op.idg : nullptr);
     else apply_update<Op::M, Op::W>(g, S, x, false);
     if (code == GM_CONVERGED || (scaled && code == GM_MAXIT)) break;
-    if (outer + 1 < g.max_restarts && !pass_end<Op::W>(y, S, 1)) return GM_SYNC;  // x is complete before it is read
+    if (outer + 1 < cycles && !pass_end<Op::W>(y, S, 1)) return GM_SYNC;  // x is complete before it is read
     code = GM_MAXIT;
   }
   if (lead(g)) g.st->gmres_iters += iters;

@@ -196,3 +196,21 @@ def test_newton_leaves_its_slopes_to_the_jacobian_operator(floors, nx, ny, preci
         out.append(sv.apply_operator("pressure_J", _known(sv, "pressure_J")))
         sv.close()
     assert rel(out[1], out[0]) <= 1e-12, rel(out[1], out[0])
+
+
+def _indefinite(nx, ny, **settings):
+    """pressure_J with slopes of both signs: not positive definite, so conjugate gradients break down."""
+    sv, prob = _solver("vortex", nx, ny, dict(B_FORM, **settings))
+    sv.prepare_operator("pressure_J", 2.0 * min(prob.dx, prob.dy))
+    sv.set_newton_state(np.where(np.arange(sv.N) % 5 == 2, -1.0, 1.0), -40.0)
+    return sv
+
+
+def test_breakdown_leaves_gmres_its_restarts():
+    """Twenty unknowns, one GMRES cycle of thirty: the cycle that the exact arithmetic solves the system in
+    is still there after conjugate gradients broke down.  Tolerance as above."""
+    sv = _indefinite(5, 4, gmres_max_restarts=1, gmres_restart=30)
+    x = _known(sv, "pressure_J")
+    got, st = sv.gmres("pressure_J", np.zeros_like(x), sv.apply_operator("pressure_J", x))
+    assert st["status"] == 0 and rel(got, x) <= 1e-8, (st, rel(got, x))
+    sv.close()
