@@ -1043,7 +1043,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
   double tol_eff = 0.0;
   int iters = 0, code = GM_MAXIT;
   const bool cg = kSym && g.kmax > 1;
-  int cycles = g.max_restarts;
+  long long cycles = g.max_restarts;
   for (int outer = 0; outer < cycles; ++outer) {
     bool ok = false;
     if constexpr (!kScalar<Op>) {
@@ -1172,7 +1172,7 @@ __device__ __forceinline__ bool pass_refine(const Op& op, const Work<float>& g, 
   return pass_end<Op::W>(y, S, 1);
 }
 template <class Op>
-__device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, double* xalt, const double* b, int max_sweeps, double tol,
+__device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, double* xalt, const double* b, long long max_sweeps, double tol,
                      Smem<Op>& smd, Sync& y) {
   const auto op32 = krylov_op<float>(op);
   using Op32 = typename std::remove_const<decltype(op32)>::type;
@@ -1222,9 +1222,10 @@ __device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, dou
       c2 = gmres_cycle(op32, g, sm, y, g.tol * res + g.tol_abs, iters);
     }
     if (c2 == GM_SYNC || c2 == GM_NONFINITE) return c2;
-    if (c2 == GM_BREAK) {  // not positive definite: GMRES from here on
+    if (c2 == GM_BREAK) {  // not positive definite: GMRES from here on, with all its sweeps
       cg = false;
       prev = INFINITY;
+      ++max_sweeps;
     }
     inner_ok = c2 == GM_CONVERGED;
     pending = true;

@@ -214,3 +214,17 @@ def test_breakdown_leaves_gmres_its_restarts():
     got, st = sv.gmres("pressure_J", np.zeros_like(x), sv.apply_operator("pressure_J", x))
     assert st["status"] == 0 and rel(got, x) <= 1e-8, (st, rel(got, x))
     sv.close()
+
+
+def test_breakdown_leaves_the_mixed_form_its_sweeps():
+    """The same in the mixed form with as many sweeps as the exact arithmetic takes."""
+    def run(**settings):
+        sv = _indefinite(5, 4, gmres_restart=30, precision="mixed", **settings)
+        x = _known(sv, "pressure_J")
+        got, st = sv.gmres("pressure_J", np.zeros_like(x), sv.apply_operator("pressure_J", x))
+        sv.close()
+        return rel(got, x), st
+    _, st = run(arith="exact")
+    assert st["status"] == 0
+    err, got = run(mixed_max_refine=st["refine_sweeps"])
+    assert got["status"] == 0 and err <= 1e-7, (st, got, err)
