@@ -1661,7 +1661,8 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   bool cg = !kRK && g.kmax > 1, faces = false, put_slopes = false;
   Smem<FaceRow<double>>& sm_faces = reinterpret_cast<Smem<FaceRow<double>>&>(smd);
   int it, iters = 0, worst = GM_CONVERGED;
-  for (it = 0; it < P.Pnewton_max; ++it) {
+  long long newton_max = P.Pnewton_max;
+  for (it = 0; it < newton_max; ++it) {
     const double* scale = scaled ? id : nullptr;
     bool ok = false;
     if constexpr (kRK) {
@@ -1734,9 +1735,10 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
         if (cg) code = cg_solve(J, g, sm, y, tol_eff, na.dp, dp_live, iters);
       }
       if (code == GM_BREAK) {
-        // not positive definite: the update so far counts as this iteration's, GMRES takes the next
+        // not positive definite: the update so far is this iteration's, which does not count; GMRES takes the next
         cg = faces = false;
         code = GM_CONVERGED;
+        ++newton_max;
       }
       for (int outer = 0; !scaled; ++outer) {
         code = gmres_cycle(J, g, sm, y, tol_eff, iters);
@@ -1773,7 +1775,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
     pending = true;
   }
   if (lead(g)) g.st->gmres_iters += iters;
-  if (it == P.Pnewton_max && lead(g)) atomicMax(&g.st->status, (int)IMEX_NEWTON_MAXIT);
+  if (it == newton_max && lead(g)) atomicMax(&g.st->status, (int)IMEX_NEWTON_MAXIT);
   // ---- the result in p; floored cells and smallest pressure (implicit_operators.cpp:722-737), and the
   // slopes of the last residual pass's iterate, which are the J mode's from here on (the reference's
   // p_freeze), unless that pass wrote them: conjugate gradients do without the plane, so it is written once

@@ -228,3 +228,24 @@ def test_breakdown_leaves_the_mixed_form_its_sweeps():
     assert st["status"] == 0
     err, got = run(mixed_max_refine=st["refine_sweeps"])
     assert got["status"] == 0 and err <= 1e-7, (st, got, err)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_breakdown_leaves_newton_its_iterations(precision):
+    """A Newton on negative enthalpies, whose Jacobian is not positive definite, with the iterations that
+    the exact arithmetic takes (a linear problem: its solution lies above the floor)."""
+    n = 6 * 5
+    x = 1.0 + 0.1 * np.random.default_rng(5).standard_normal(n)
+    cold = np.arange(0, n, 7)
+    need = None
+    for arith in ("exact", "fast"):
+        more = {} if need is None else dict(Pnewton_max=need)
+        sv = _newton_solver(6, 5, 2.0, arith=arith, precision=precision, gmres_restart=30, p_floor=1e-3, **more)
+        q = sv.cons()
+        q[4].reshape(-1)[cold] -= 40.0
+        sv.set_buffer("Qe", q)
+        sv.prepare_operator("pressure_L", 2.0 * 10.0 / 6)
+        p, st = sv.nested_newton(np.full(n, 0.9), sv.apply_operator("pressure_L", x))
+        assert st["status"] == 0 and rel(p, x) <= 1e-7, (arith, st, rel(p, x))
+        need = st["newton_iters"] + 1  # the last iteration finds the residual small
+        sv.close()
