@@ -860,14 +860,19 @@ imex_status amalloc(Adj& W, double** p, size_t count) {
   *p = static_cast<double*>(q);
   return IMEX_OK;
 }
+// What a context keeps between calls, of the workspace and of the checkpoints each, is at most this: a
+// grid of about 280^2.  An allocation and its release cost a millisecond, and up to 100 on a busy host,
+// beside a call of 22 ms on 128^2; from here on a call takes longer than that, and the gigabytes are worth
+// more to the program's other contexts (some 400 planes: 840 MB on 512^2, 13 GB on 2048^2).
+constexpr size_t kKeepBytes = size_t(256) << 20;
 // one allocation for `states` checkpoints (13 planes each) and the planes of the outputs
 imex_status state_slab(Adj& W, size_t states) {
   const size_t N = W.N, bytes = states * (block_bytes(8 * N) + 2 * block_bytes(N) + block_bytes(3 * N)) +
                                 2 * block_bytes(8 * N) + block_bytes(N) + block_bytes(3 * N);
   imex_ctx* ctx = W.ctx;
-  // a slab no larger than the workspace stays with the context too (an allocation and its release
-  // cost up to 100 ms on a busy host); a long run's checkpoints are given back with the call
-  const bool keep = bytes <= ctx->adj_ws_bytes;
+  // a slab no larger than a kept workspace stays with the context too; a long run's checkpoints are
+  // given back with the call
+  const bool keep = bytes <= ctx->adj_ws_bytes && bytes <= kKeepBytes;
   void* q = nullptr;
   if (keep && ctx->adj_slab && ctx->adj_slab_bytes >= bytes) {
     q = ctx->adj_slab;
@@ -893,6 +898,10 @@ imex_status state_slab(Adj& W, size_t states) {
 void afree(Adj& W) {
   for (void* p : W.mem) cudaFree(p);
   W.mem.clear();
+  if (W.ctx->adj_ws_bytes <= kKeepBytes) return;
+  cudaFree(W.ctx->adj_ws);
+  W.ctx->adj_ws = nullptr;
+  W.ctx->adj_ws_bytes = 0;
 }
 imex_status zero(Adj& W, double* p, size_t count) {
   return cuda_check(W.ctx, cudaMemsetAsync(p, 0, count * sizeof(double), W.ctx->stream), "adjoint clear");
@@ -914,9 +923,8 @@ imex_status put_sc(imex_ctx* ctx, const DevScalars& in) {
   return cuda_check(ctx, e, "adjoint scalars");
 }
 
-// The planes of the reverse sweep.  Their number depends on the context alone (grid, stages,
-// Energy_Modify), so the context keeps them from call to call, in one allocation, until it is
-// destroyed: with about 150 separate allocations per call a three-step product on 128^2 took
+// The planes of the reverse sweep, in one allocation.  Their number depends on the context alone (grid,
+// stages, Energy_Modify), so the context keeps them from call to call up to kKeepBytes: with about 150 separate allocations per call a three-step product on 128^2 took
 // 48.6 ms (and 50 to 160 when the driver's allocator was slow), with these kept 29.3.
 imex_status workspace(Adj& W) {
   imex_ctx* ctx = W.ctx;
@@ -947,7 +955,7 @@ imex_status workspace(Adj& W) {
   for (const auto& q : want) bytes += block_bytes(q.second);
   if (!ctx->adj_ws) {
     cudaError_t e = cudaMalloc(&ctx->adj_ws, bytes);
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->adj_host, 16 * sizeof(double));
+    if (e == cudaSuccess && !ctx->adj_host) e = cudaMallocHost(&ctx->adj_host, 16 * sizeof(double));
     if (e != cudaSuccess) {
       cudaFree(ctx->adj_ws);
       ctx->adj_ws = nullptr;

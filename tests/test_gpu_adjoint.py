@@ -191,3 +191,31 @@ def test_adjoint_rejects_unsupported_configurations():
             sv.adjoint_run(1, prob.prim[0], prob.prim[5:8])
         assert err.value.status == 2
         sv.close()
+
+
+def test_a_large_adjoint_gives_its_memory_back():
+    """What a context keeps after a call is at most 256 MiB of workspace and as much of checkpoints (the
+    512^2 workspace has about 840 MB); a second call gives the same result to the rounding of its atomic sums."""
+    import torch
+
+    def product(sv, n):
+        lam = np.random.default_rng(1).standard_normal((8, n, n))
+        return sv.adjoint_vjp(1, lam, checkpoint_every=1)
+
+    small = ix.Solver.for_problem(vortex(64), 2, CFG)
+    product(small, 64)  # the kernels are loaded, with their local memory
+    sv = ix.Solver.for_problem(vortex(512), 2, CFG)
+    sv.step()
+    sv.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    sv.load(vortex(512))
+    first = product(sv, 512)
+    held = before - torch.cuda.mem_get_info()[0]
+    assert held <= 520 * 2**20, held / 2**20
+    sv.load(vortex(512))
+    second = product(sv, 512)
+    for a, b in zip(first, second):
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(a)
+    assert before - torch.cuda.mem_get_info()[0] <= 520 * 2**20
+    sv.close()
+    small.close()
