@@ -2680,7 +2680,6 @@ imex_status gmres_noalloc_march(imex_ctx* ctx, int op, double* x, const double* 
   if (e != cudaSuccess) return cuda_check(ctx, e, "imex_gmres_noalloc: vector upload");
   imex_status s = march::gmres_solve(ctx, op, gmres_family(op), xd, bd, &w);
   if (s != IMEX_OK) return s;
-  ctx->kernel_launches += ctx->prof_on ? 0 : 1;
   if (hx) e = cudaMemcpyAsync(x, xd, n * sizeof(double), cudaMemcpyDefault, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   return cuda_check(ctx, e, "imex_gmres_noalloc: solve");

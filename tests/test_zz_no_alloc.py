@@ -74,3 +74,17 @@ def test_noalloc_rejects_oversize_solve_and_context_survives():
     x, st = sv.gmres("magnetic_B", x0, b)
     assert st["status"] == 0 and np.isfinite(x).all()
     sv.close()
+
+
+@pytest.mark.parametrize("op,factory,rks,settings", CASES)
+@pytest.mark.parametrize("profiled", [False, True])
+def test_noalloc_counts_the_kernels_of_imex_gmres(op, factory, rks, settings, profiled):
+    """The two calls launch the same kernels, so imex_kernel_launch_count grows alike."""
+    sv, x0, b = _prepared(op, factory, rks, settings)
+    sv.profile_enable(profiled)
+    counts = [sv.kernel_launches()]
+    for solve in (sv.gmres, sv.gmres_noalloc):
+        solve(op, x0, b)
+        counts.append(sv.kernel_launches())
+    assert counts[2] - counts[1] == counts[1] - counts[0] > 0, counts
+    sv.close()
