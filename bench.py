@@ -398,7 +398,7 @@ def run_ensemble(args, world: int, rank: int, local: int) -> None:
         launches_per_step = info["explicit_launches_per_step"] + info["planned_solve_launches_per_step"]
     else:
         launches_per_step = (sum(m.kernel_launches() for m in batch.members) - launches0
-                             + 2 * info["solve_launches_per_step"])
+                             + info["solve_launches_per_step"])
     for _ in range(max(args.warmup - 1, 2)):
         batch.step(1)
     cells_per_step = sum(p.nx * p.ny for p in probs) * wl["rks"]

@@ -527,10 +527,11 @@ imex_status imex_batch_explicit_launches(imex_batch* b, int* launches_per_step, 
     for (const PlanItem& it : b->plan) n += it.solve < 0 ? 1 : 0;
   }
   *launches_per_step = n;
-  if (solve_launches_per_step) {  // a chunk of a batched solve: a barrier reset and the solve
+  if (solve_launches_per_step) {
     int m = 0;
     for (const PlanItem& it : b->plan)
-      if (it.solve >= 0) m += 2 * (int)solve_plan(b, it.solve)->chunks.size();
+      if (it.solve >= 0)
+        for (const BatchChunk& ch : solve_plan(b, it.solve)->chunks) m += ch.kernels;
     *solve_launches_per_step = b->nstreams == 0 ? m : -1;
   }
   return IMEX_OK;

@@ -257,8 +257,8 @@ imex_status run_barrier_selftest(imex_ctx* ctx, int iterations, int phantom_bloc
 // as cooperative launches in which each member owns a contiguous range of CTAs
 enum { BATCH_MAGNETIC = 0, BATCH_PRESSURE = 1 };
 struct BatchChunk {
-  std::function<cudaError_t(cudaStream_t)> launch;  // barrier reset + the cooperative launch
-  int ctas = 0, members = 0;
+  std::function<cudaError_t(cudaStream_t)> launch;  // the cooperative launch, and a tile solve's barrier reset
+  int ctas = 0, members = 0, kernels = 1;
 };
 struct BatchSolvePlan {
   std::vector<BatchChunk> chunks;

@@ -2803,6 +2803,7 @@ imex_status add_chunks(BatchSolvePlan* plan, const std::vector<imex_ctx*>& membe
     BatchChunk ch;
     ch.ctas = nctas;
     ch.members = n;
+    ch.kernels = 2;
     ch.launch = [=](cudaStream_t st) {
       k_reset_syncs<<<(n + 255) / 256, 256, 0, st>>>(d_syncs, n, limit);
       cudaError_t e2 = cudaGetLastError();

@@ -411,8 +411,8 @@ imex_status imex_batch_configure(imex_batch* b, int streams, int use_graph);
 /* advance every member `steps` steps; *device_ms (optional) = device time of those steps */
 imex_status imex_batch_step(imex_batch* b, int steps, double* device_ms);
 /* launches of one ensemble step in the batched mode: the explicit sub-steps, and the
- * batched solves (a barrier reset and a cooperative launch per chunk); -1 in the streams
- * mode.  The second pointer may be null. */
+ * batched solves (a cooperative launch per chunk, with a barrier reset before it in the tile
+ * kernels); -1 in the streams mode.  The second pointer may be null. */
 imex_status imex_batch_explicit_launches(imex_batch* b, int* launches_per_step, int* solve_launches_per_step);
 /* tile shape of the batched B-form magnetic solve in the fast arithmetic: 0 = 32 x 16 cells
  * (the default, and the shape of every single-context solve), 1 = 64 x 8, 2 = 32 x 8 */

@@ -129,3 +129,17 @@ def test_batch_solve_tile_shapes_match_single_runs(tile):
     batch.step(2)
     _check_members(batch, probs, 2, CFG0, 2, 1e-11, 1e-10)
     batch.close()
+
+
+@pytest.mark.parametrize("glf,kernels", [(1, 1), (0, 2)])
+def test_batch_counts_the_launches_of_its_solves(glf, kernels):
+    """Three members fit one chunk a solve.  An RK2 step solves the magnetic system once a stage and the
+    pressure once or twice: with the marching kernels (global dissipation) one launch each, with the tile
+    kernels (local dissipation) a barrier reset and a launch."""
+    batch = ix.Batch(_members()[:3], 2, dict(CFG0, GLF=glf))
+    batch.step(1)
+    info = batch.info()
+    assert info["solve_launches_per_step"] == 2  # the chunks of the two plans
+    solves = info["planned_solve_launches_per_step"] / kernels
+    assert solves in (4, 5, 6), info
+    batch.close()
