@@ -414,12 +414,14 @@ imex_status imex_batch_step(imex_batch* b, int steps, double* device_ms);
  * batched solves (a cooperative launch per chunk, with a barrier reset before it in the tile
  * kernels); -1 in the streams mode.  The second pointer may be null. */
 imex_status imex_batch_explicit_launches(imex_batch* b, int* launches_per_step, int* solve_launches_per_step);
-/* tile shape of the batched B-form magnetic solve in the fast arithmetic: 0 = 32 x 16 cells
- * (the default, and the shape of every single-context solve), 1 = 64 x 8, 2 = 32 x 8 */
+/* tile shape of the batched B-form magnetic solve in the fast arithmetic with local dissipation
+ * (GLF = 0): 0 = 32 x 16 cells (the default, and the shape of every single-context tile solve),
+ * 1 = 64 x 8, 2 = 32 x 8.  Without effect where the row-marching kernels solve (GLF = 1), which
+ * have no tiles. */
 imex_status imex_batch_set_solve_tile(imex_batch* b, int tile);
 /* time `trial_steps` ensemble steps per candidate, one choice at a time from the best so
  * far: the explicit mode (batched launches, or 4 / 8 / 16 streams), the B-form solve's tile
- * shape (B form, fast arithmetic), the restart length (15 or the configured one) and, in
+ * shape (where imex_batch_set_solve_tile has effect), the restart length (15 or the configured one) and, in
  * mixed precision, the configured mixed_solves or the same with the magnetic systems' FP32
  * form toggled; restore every member's state after each trial and keep the fastest */
 imex_status imex_batch_autotune(imex_batch* b, int trial_steps, imex_batch_tuning* out);

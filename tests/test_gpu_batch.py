@@ -143,3 +143,16 @@ def test_batch_counts_the_launches_of_its_solves(glf, kernels):
     solves = info["planned_solve_launches_per_step"] / kernels
     assert solves in (4, 5, 6), info
     batch.close()
+
+
+@pytest.mark.parametrize("tile", [1, 2])
+def test_batch_solve_tile_shapes_of_the_local_dissipation(tile):
+    """The 64x8 and 32x8 tiles where they run: the fast B form with local dissipation, whose solves the
+    marching kernels do not take.  Tolerances as for the 32x16 tiles above."""
+    probs = _members()[:3]
+    settings = dict(CFG0, GLF=0, add_pvisc="AlfvenSpeedp")
+    batch = ix.Batch(probs, 2, settings)
+    batch.set_solve_tile(tile)
+    batch.step(2)
+    _check_members(batch, probs, 2, settings, 2, 1e-11, 1e-10)
+    batch.close()
