@@ -3,8 +3,8 @@
 ``build_library()`` compiles every CUDA source of imex_b200/csrc with nvcc for
 sm_100a into ``imex_b200/libimex_b200.so`` (in-tree, so it travels with the
 repository snapshot).  FMA contraction is disabled (``-fmad=false``) so that
-the FP64 kernels round exactly like the reference's x86 build, except in the
-row-marching solver kernels (FMAD), whose results are a solve's to its tolerance.
+the FP64 kernels round exactly like the reference's x86 build, except in the row-marching
+solver kernels of the sources in FMAD, whose results are a solve's to its tolerance.
 """
 from __future__ import annotations
 

@@ -93,8 +93,10 @@ __device__ __forceinline__ T left1(T v) {
 //         a thread, 12 have 168).  Measured: the ideal gas's pressure at 12 and 16 warps, with
 //         spills, 11 and 35 % slower on 251 x 173; the B form at 12, 30 % slower on 768^2; the
 //         Redlich-Kwong residual, compute bound, 3 % faster at 12 than at 8,
-//   K     Krylov vectors whose loads for a row are in flight together,
-//   completed rows per round of dot products (their vectors are still in the L1),
+//   R     FP64 vectors of a row that the ring in shared memory holds (Ring; twice as many in FP32),
+//   kDots   vectors whose dot products a lane sums in registers over its rows (the others' are added
+//         across the warp at every row),
+//   kAhead  vectors past the ring whose row is loaded ahead of its use, into registers,
 //   step(st, w, in, em, out, wc): takes the arriving row w, completes the row H below it:
 //         out = A w there, wc = w there.
 // precond applies the solve's Jacobi preconditioner to a completed row (it uses the diagonal
@@ -742,7 +744,7 @@ struct Shared {
   double H[kCap + 2][kCap + 2];                // rotated Hessenberg columns
   double hcol[kCap + 2], coef[kCap + 2];       // the current raw column; an update's weights
   double comb[kCap + 3];                       // weights of the terms of the next vector
-  double cs[kCap + 2], sn[kCap + 2], gam[kCap + 2], alpha[kCap + 2], sigma[kCap + 2];
+  double cs[kCap + 2], sn[kCap + 2], gam[kCap + 2], sigma[kCap + 2];
   double red[kSlots];
   double acc[kMaxWarps][kSlots];
   double cga[kCap + 2], cgb[kCap + 2];         // conjugate gradients: alpha_k, beta_k
@@ -750,8 +752,6 @@ struct Shared {
   int cycles;  // of this solve, counted by its first block
   double bytes;
 };
-
-enum { RED_SUM = 0, RED_MIN = 1 };
 
 struct Sync {
   SyncState* s;

@@ -15,10 +15,10 @@
 // on middle grids, and on small grids the pass end.  The tile kernels (kernels_solve.cu), which
 // keep the configurations these do not take, stage 32 x 16 tiles in shared memory with two or
 // three block barriers per tile and were latency bound at 24-33 % of the issue slots.  Measured
-// against them, us per solve: A form 1024^2 429 -> 277, 2048^2 1520 -> 919; B form 768^2 (Krylov
-// spaces of 25) 2533 -> 1966, open 700 x 450 900 -> 553, 320^2 296 -> 210; nested Newton 64^2 131 -> 90, 700 x 450 348 ->
-// 148, 1024^2 326 -> 169, 2048^2 1189 -> 670, Redlich-Kwong 768^2 689 -> 411; one pressure solve
-// of 75 steps on 513 x 400 1609 -> 620.
+// against them, us per solve: A form 1024^2 429 -> 277, 2048^2 1520 -> 909; B form 768^2 (Krylov
+// spaces of 25) 2533 -> 1963, open 700 x 450 900 -> 555, 320^2 296 -> 212; nested Newton 64^2 131 -> 87,
+// 700 x 450 348 -> 152, 1024^2 326 -> 151, 2048^2 1189 -> 491, Redlich-Kwong 768^2 689 -> 412; one
+// pressure solve of 75 steps on 513 x 400 1609 -> 640.
 #pragma once
 
 #include <algorithm>
@@ -599,8 +599,8 @@ __device__ __forceinline__ bool pass_residual(const Op& op, const Work<TS>& g, S
 
 // ------------------------------------------------------------------ one GMRES cycle
 // From V0 = r0 (left-preconditioned residual, norm S.gam[0] > tol): up to kmax Arnoldi steps,
-// the Givens update of each column and the back substitution.  Leaves S.alpha[i] * S.sigma[i]
-// in S.coef[0, S.nalpha), the weights of the update sum_i coef_i V_i.
+// the Givens update of each column and the back substitution.  Leaves the weights of the
+// update sum_i coef_i V_i in S.coef[0, S.nalpha).
 template <class Op, class TS>
 __device__ __forceinline__ int gmres_cycle(const Op& op, const Work<TS>& g, Smem<Op>& sm, Sync& y, double tol_eff, int& iters) {
   Shared& S = sm.S;
@@ -677,7 +677,6 @@ __device__ __forceinline__ int gmres_cycle(const Op& op, const Work<TS>& g, Smem
       if (tid == k) yv = ak;
     }
     if (tid <= jend) {
-      S.alpha[tid] = yv;
       S.coef[tid] = yv * S.sigma[tid];
     }
     if (tid == 0) {
@@ -741,7 +740,6 @@ struct StagedRows {
     rows = (ya + G.L < G.ny ? ya + G.L : G.ny) - ya;
   }
   __device__ __forceinline__ int count() const { return rows + 2; }
-  __device__ __forceinline__ bool inner(int it) const { return it >= 1 && it <= rows; }  // the task's own rows
   template <class Copy>
   __device__ __forceinline__ void issue(int it, Copy& copy) const {
     if (it < rows + 2) {
