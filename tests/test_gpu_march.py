@@ -249,3 +249,22 @@ def test_breakdown_leaves_newton_its_iterations(precision):
         assert st["status"] == 0 and rel(p, x) <= 1e-7, (arith, st, rel(p, x))
         need = st["newton_iters"] + 1  # the last iteration finds the residual small
         sv.close()
+
+
+@pytest.mark.parametrize("kind", ["vortex", "blast"])
+@pytest.mark.parametrize("op,settings", [("pressure_L", B_FORM), ("energy", ENERGY)])
+@pytest.mark.parametrize("h", [4.0, 16.0])
+def test_march_long_solves_are_as_accurate_as_gmres(op, settings, kind, h):
+    """Solves of a hundred steps and more (condition numbers of 1e3 to 1e5): conjugate gradients stop on their
+    recurrence residual however many they take, restarted GMRES (the exact arithmetic) forms b - A x at every
+    restart.  The error is no larger than GMRES's, whose residual meets the same tolerance."""
+    err = []
+    for arith in ("exact", "fast"):
+        sv, prob = _solver(kind, 64, 63, dict(settings, arith=arith))
+        sv.prepare_operator(op, h * min(prob.dx, prob.dy))
+        x = 1.0 + 0.3 * _known(sv, op)
+        got, st = sv.gmres(op, np.zeros_like(x), sv.apply_operator(op, x))
+        assert st["status"] == 0 and st["gmres_iters"] > 100, st
+        err.append(rel(got, x))
+        sv.close()
+    assert err[1] <= err[0], err
