@@ -1067,7 +1067,9 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
         bool live = true;
         code = cg_solve(kop, g, sm, y, tol_eff, x, live, iters);
         scaled = true;
-        if (code == GM_BREAK) ++cycles;  // GMRES has all of its own
+        // where they break down, or need more steps than GMRES may (it minimises the norm that is tested,
+        // and can end a few steps before them), GMRES goes on from here with all its restarts
+        if (code == GM_BREAK || code == GM_MAXIT) ++cycles;
       }
     }
     if (!scaled) {
@@ -1078,7 +1080,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
     if (code == GM_SYNC || code == GM_NONFINITE) break;
     if constexpr (kSym) apply_update<Op::M, Op::W>(g, S, x, false, scaled ? op.idg : nullptr);
     else apply_update<Op::M, Op::W>(g, S, x, false);
-    if (code == GM_CONVERGED || (scaled && code == GM_MAXIT)) break;
+    if (code == GM_CONVERGED) break;
     if (outer + 1 < cycles && !pass_end<Op::W>(y, S, 1)) return GM_SYNC;  // x is complete before it is read
     code = GM_MAXIT;
   }

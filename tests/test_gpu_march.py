@@ -268,3 +268,21 @@ def test_march_long_solves_are_as_accurate_as_gmres(op, settings, kind, h):
         err.append(rel(got, x))
         sv.close()
     assert err[1] <= err[0], err
+
+
+@pytest.mark.parametrize("op,settings", [("pressure_L", B_FORM), ("energy", ENERGY)])
+@pytest.mark.parametrize("kind,nx,ny,restart", [("vortex", 6, 5, 30), ("blast", 5, 6, 30), ("blast", 63, 41, 2)])
+def test_a_cap_that_gmres_stays_below_is_no_refusal(op, settings, kind, nx, ny, restart):
+    """Conjugate gradients can need a few steps more than GMRES, which minimises the residual's norm: a solve
+    with as many restarts as the exact arithmetic takes still ends.  Thirty unknowns are one cycle of thirty.
+    Tolerance: the stopping tolerance 1e-13 times the condition number, below 1e5."""
+    need, steps = None, 30.0 if nx < 30 else 1.0
+    for arith in ("exact", "fast"):
+        more = {} if need is None else dict(gmres_max_restarts=need)
+        sv, prob = _solver(kind, nx, ny, dict(settings, arith=arith, gmres_restart=restart, **more))
+        sv.prepare_operator(op, steps * min(prob.dx, prob.dy))
+        x = _known(sv, op)
+        got, st = sv.gmres(op, np.zeros_like(x), sv.apply_operator(op, x))
+        assert st["status"] == 0 and rel(got, x) <= 1e-8, (arith, need, st, rel(got, x))
+        need = st["gmres_restarts"]
+        sv.close()
