@@ -1734,8 +1734,9 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       if constexpr (!kRK) {
         if (cg) code = cg_solve(J, g, sm, y, tol_eff, na.dp, dp_live, iters);
       }
-      if (code == GM_BREAK) {
-        // not positive definite: the update so far is this iteration's, which does not count; GMRES takes the next
+      if (scaled && (code == GM_BREAK || code == GM_MAXIT)) {
+        // not positive definite, or more steps than GMRES may take: the update so far is this iteration's, which
+        // does not count; GMRES takes the next
         cg = faces = false;
         code = GM_CONVERGED;
         ++newton_max;

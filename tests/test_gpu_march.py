@@ -286,3 +286,15 @@ def test_a_cap_that_gmres_stays_below_is_no_refusal(op, settings, kind, nx, ny, 
         assert st["status"] == 0 and rel(got, x) <= 1e-8, (arith, need, st, rel(got, x))
         need = st["gmres_restarts"]
         sv.close()
+
+
+@pytest.mark.parametrize("steps", [10.0, 30.0, 100.0])
+def test_a_cap_that_newtons_gmres_stays_below_is_no_refusal(steps):
+    """The same for the Jacobian solves of the nested Newton (a linear problem, solution above the floor)."""
+    for arith in ("exact", "fast"):
+        sv, prob = _solver("blast", 5, 6, dict(B_FORM, arith=arith, gmres_restart=30, gmres_max_restarts=1, p_floor=1e-6))
+        sv.prepare_operator("pressure_L", steps * min(prob.dx, prob.dy))
+        x = 1.0 + 0.1 * _known(sv, "pressure_L")
+        p, st = sv.nested_newton(np.full(sv.N, 0.9), sv.apply_operator("pressure_L", x))
+        assert st["status"] == 0 and rel(p, x) <= 1e-6, (arith, st, rel(p, x))
+        sv.close()
