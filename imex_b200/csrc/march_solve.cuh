@@ -1114,8 +1114,9 @@ __global__ void __launch_bounds__(32 * Op::W, 1) k_gmres_jobs(const GmresJob<Op>
 //   x <- x + (pending inner update), s = b - A x, r0 = M^-1 s stored in FP32, |r0|,
 // which stops at |r0| <= tol |r0 of the first sweep| + tol, or at the FP64 rounding floor (an
 // inner cycle met its tolerance and yet the residual fell by less than half, or two sweeps in
-// a row fell by less than half), and one FP32 cycle on M^-1 A d = r0, stopped at a relative
-// residual of g.tol or after kmax steps.  x is double buffered between x and xalt.
+// a row fell by less than half), and one FP32 GMRES cycle on M^-1 A d = r0, stopped at a relative
+// residual of g.tol or after kmax steps (the symmetric systems: conjugate gradients to that
+// residual).  x is double buffered between x and xalt.
 template <class Op>
 struct MixedJob {
   Op op;
@@ -1213,7 +1214,9 @@ __device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, dou
     if (lead(g)) g.st->refine_sweeps += 1;
     int c2 = GM_MAXIT;
     scaled = cg;
-    if constexpr (kSymmetric<Op>) {  // one cycle, so x is not touched before the next sweep
+    if constexpr (kSymmetric<Op>) {
+      // to the inner tolerance, full slots added to the iterate: cut off after one cycle as GMRES is, the sweeps
+      // of an ill-conditioned system gain too little to end within their cap
       if (cg) c2 = cg_solve(op32, g, sm, y, g.tol * res + g.tol_abs, xc, x_live, iters);
     }
     if (!scaled) {
@@ -2011,7 +2014,6 @@ imex_status solve(imex_ctx* ctx, bool jac, int fam, int kind, double* x, const d
     j.op = make_op<MOp>(ctx, jac);
     j.g = make_work<float>(ctx, k, MOp::M, fam);
     j.g.tol_abs = 0.0;
-    j.g.max_restarts = 1;
     j.x = x;
     j.xalt = ctx->mcor;
     j.b = b;
@@ -2141,7 +2143,6 @@ imex_status add_solves(BatchSolvePlan* plan, const std::vector<imex_ctx*>& membe
     j.op = make_op<MOp>(m);
     j.g = make_work<float>(m, k, MOp::M, fam);
     j.g.tol_abs = 0.0;
-    j.g.max_restarts = 1;
     system(m, &j.x, &j.b);
     j.xalt = m->mcor;
     j.max_sweeps = m->cfg.mixed_max_refine;

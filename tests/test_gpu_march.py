@@ -298,3 +298,18 @@ def test_a_cap_that_newtons_gmres_stays_below_is_no_refusal(steps):
         p, st = sv.nested_newton(np.full(sv.N, 0.9), sv.apply_operator("pressure_L", x))
         assert st["status"] == 0 and rel(p, x) <= 1e-6, (arith, st, rel(p, x))
         sv.close()
+
+
+@pytest.mark.parametrize("kind", ["vortex", "blast"])
+@pytest.mark.parametrize("op,settings", [("pressure_L", B_FORM), ("energy", ENERGY)])
+@pytest.mark.parametrize("restart", [2, 5, 12, 25])
+def test_march_mixed_form_refines_ill_conditioned_systems(op, settings, kind, restart):
+    """The mixed form within its fifty sweeps, however few residuals the inner solves keep.  Tolerance:
+    mixed_outer_tol = 1e-10 times a condition number below 1e4."""
+    for steps in (3.0, 10.0):
+        sv, prob = _solver(kind, 143, 109, dict(settings, precision="mixed", mixed_solves=7, gmres_restart=restart))
+        sv.prepare_operator(op, steps * min(prob.dx, prob.dy))
+        x = _known(sv, op)
+        got, st = sv.gmres(op, np.zeros_like(x), sv.apply_operator(op, x))
+        assert st["status"] == 0 and rel(got, x) <= 1e-6, (steps, st, rel(got, x))
+        sv.close()
