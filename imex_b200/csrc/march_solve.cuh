@@ -1665,6 +1665,8 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   Smem<FaceRow<double>>& sm_faces = reinterpret_cast<Smem<FaceRow<double>>&>(smd);
   int it, iters = 0, worst = GM_CONVERGED;
   long long newton_max = P.Pnewton_max;
+  constexpr int kMore = 3;
+  int more = 0;
   for (it = 0; it < newton_max; ++it) {
     const double* scale = scaled ? id : nullptr;
     bool ok = false;
@@ -1703,7 +1705,15 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       worst = GM_NONFINITE;
       break;
     }
-    if (res < P.Pnewton_tol * res0 + P.Pnewton_tol) break;
+    if (res < P.Pnewton_tol * res0 + P.Pnewton_tol) {
+      // The FP32 solves can leave the residual just below the tolerance, and the tolerance can leave a pressure
+      // below a floor smaller than itself, where an FP64 solve has gone far beyond: further iterations then,
+      // at most kMore, before that counts as IMEX_POSITIVITY.
+      if (!std::is_same<TS, float>::value || !P.floor_on || !(S.red[3] < P.theta * P.p_floor - 1e-14) || more >= kMore ||
+          it + 1 >= newton_max)
+        break;
+      ++more;
+    }
     // ---- Jacobian solve J dp = -g (GMRES with precP) from dp = 0
     if (lead(g)) {
       g.st->gmres_solves += 1;
