@@ -729,8 +729,9 @@ __device__ __forceinline__ void arrive(unsigned long long* p) {
   asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(p) : "memory");
 }
 constexpr unsigned long long kGaveUp = 1ull << 63;
-// gives the launch up unless the target has been reached in the meantime; the counter as decided
-__device__ __forceinline__ unsigned long long give_up(unsigned long long* p, unsigned long long target) {
+// gives the launch up unless the target has been reached in the meantime; the counter as decided (called:
+// inlined it costs the B-form solve 16 bytes of spills, and its steps half a percent)
+static __device__ __noinline__ unsigned long long give_up(unsigned long long* p, unsigned long long target) {
   unsigned long long v = ld_relaxed(p);
   while (v < target) {
     const unsigned long long was = atomicCAS(p, v, v | kGaveUp);

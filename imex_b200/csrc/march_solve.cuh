@@ -1041,8 +1041,8 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
   double tol_eff = 0.0;
   int iters = 0, code = GM_MAXIT;
   const bool cg = kSym && g.kmax > 1;
-  long long cycles = g.max_restarts;
-  for (int outer = 0; outer < cycles; ++outer) {
+  int free = 0;  // cycles that do not count
+  for (int outer = 0; outer - free < g.max_restarts; ++outer) {
     bool ok = false;
     if constexpr (!kScalar<Op>) {
       ok = pass_residual<false>(op, g, S, y, x, b);
@@ -1069,7 +1069,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
         scaled = true;
         // where they break down, or need more steps than GMRES may (it minimises the norm that is tested,
         // and can end a few steps before them), GMRES goes on from here with all its restarts
-        if (code == GM_BREAK || code == GM_MAXIT) ++cycles;
+        if (code == GM_BREAK || code == GM_MAXIT) free = 1;
       }
     }
     if (!scaled) {
@@ -1081,7 +1081,7 @@ __device__ __forceinline__ int gmres(const Op& op, const Work<double>& g, double
     if constexpr (kSym) apply_update<Op::M, Op::W>(g, S, x, false, scaled ? op.idg : nullptr);
     else apply_update<Op::M, Op::W>(g, S, x, false);
     if (code == GM_CONVERGED) break;
-    if (outer + 1 < cycles && !pass_end<Op::W>(y, S, 1)) return GM_SYNC;  // x is complete before it is read
+    if (outer + 1 - free < g.max_restarts && !pass_end<Op::W>(y, S, 1)) return GM_SYNC;  // x is complete before it is read
     code = GM_MAXIT;
   }
   if (lead(g)) g.st->gmres_iters += iters;
@@ -1173,7 +1173,7 @@ __device__ __forceinline__ bool pass_refine(const Op& op, const Work<float>& g, 
   return pass_end<Op::W>(y, S, 1);
 }
 template <class Op>
-__device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, double* xalt, const double* b, long long max_sweeps, double tol,
+__device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, double* xalt, const double* b, int max_sweeps, double tol,
                      Smem<Op>& smd, Sync& y) {
   const auto op32 = krylov_op<float>(op);
   using Op32 = typename std::remove_const<decltype(op32)>::type;
@@ -1182,7 +1182,7 @@ __device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, dou
   double *xc = x, *xn = xalt;
   bool pending = false, inner_ok = false, scaled = false, x_live = true;
   bool cg = kSymmetric<Op> && g.kmax > 1;
-  int stalls = 0, iters = 0, code = GM_MAXIT;
+  int stalls = 0, iters = 0, code = GM_MAXIT, free = 0;  // free: sweeps that do not count
   double tol_eff = 0.0, prev = INFINITY;
   for (int sweep = 0;; ++sweep) {
     const double* scale = nullptr;
@@ -1210,7 +1210,7 @@ __device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, dou
       break;
     }
     prev = res;
-    if (sweep >= max_sweeps) break;
+    if (sweep - free >= max_sweeps) break;
     if (lead(g)) g.st->refine_sweeps += 1;
     int c2 = GM_MAXIT;
     scaled = cg;
@@ -1228,7 +1228,7 @@ __device__ __forceinline__ int mixed(const Op& op, Work<float> g, double* x, dou
     if (c2 == GM_BREAK) {  // not positive definite: GMRES from here on, with all its sweeps
       cg = false;
       prev = INFINITY;
-      ++max_sweeps;
+      free = 1;
     }
     inner_ok = c2 == GM_CONVERGED;
     pending = true;
@@ -1664,10 +1664,10 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
   bool cg = !kRK && g.kmax > 1, faces = false, put_slopes = false;
   Smem<FaceRow<double>>& sm_faces = reinterpret_cast<Smem<FaceRow<double>>&>(smd);
   int it, iters = 0, worst = GM_CONVERGED;
-  long long newton_max = P.Pnewton_max;
+  int free = 0;  // iterations that do not count
   constexpr int kMore = 3;
   int more = 0;
-  for (it = 0; it < newton_max; ++it) {
+  for (it = 0; it - free < P.Pnewton_max; ++it) {
     const double* scale = scaled ? id : nullptr;
     bool ok = false;
     if constexpr (kRK) {
@@ -1710,7 +1710,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
       // below a floor smaller than itself, where an FP64 solve has gone far beyond: further iterations then,
       // at most kMore, before that counts as IMEX_POSITIVITY.
       if (!std::is_same<TS, float>::value || !P.floor_on || !(S.red[3] < P.theta * P.p_floor - 1e-14) || more >= kMore ||
-          it + 1 >= newton_max)
+          it + 1 - free >= P.Pnewton_max)
         break;
       ++more;
     }
@@ -1752,7 +1752,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
         // does not count; GMRES takes the next
         cg = faces = false;
         code = GM_CONVERGED;
-        ++newton_max;
+        free = 1;
       }
       for (int outer = 0; !scaled; ++outer) {
         code = gmres_cycle(J, g, sm, y, tol_eff, iters);
@@ -1789,7 +1789,7 @@ __device__ __forceinline__ int newton(const PressureRow<double, kRK>& op, Work<T
     pending = true;
   }
   if (lead(g)) g.st->gmres_iters += iters;
-  if (it == newton_max && lead(g)) atomicMax(&g.st->status, (int)IMEX_NEWTON_MAXIT);
+  if (it - free == P.Pnewton_max && lead(g)) atomicMax(&g.st->status, (int)IMEX_NEWTON_MAXIT);
   // ---- the result in p; floored cells and smallest pressure (implicit_operators.cpp:722-737), and the
   // slopes of the last residual pass's iterate, which are the J mode's from here on (the reference's
   // p_freeze), unless that pass wrote them: conjugate gradients do without the plane, so it is written once
