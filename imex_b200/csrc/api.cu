@@ -115,7 +115,8 @@ imex_status dalloc(imex_ctx* ctx, T** p, size_t count) {
   cudaError_t e = cudaMalloc(&q, count * sizeof(T) > 0 ? count * sizeof(T) : 8);
   if (e != cudaSuccess) return cuda_check(ctx, e, "cudaMalloc");
   ctx->allocations.push_back(q);
-  e = cudaMemset(q, 0, count * sizeof(T));
+  // on the context's stream, which does not wait for the default one: the solves' counters start from zero
+  e = cudaMemsetAsync(q, 0, count * sizeof(T), ctx->stream);
   if (e != cudaSuccess) return cuda_check(ctx, e, "cudaMemset");
   *p = static_cast<T*>(q);
   return IMEX_OK;
