@@ -2078,9 +2078,16 @@ imex_status newton_one(imex_ctx* ctx, double* p, const double* b, int keys) {
 }
 
 // ---- ensembles: one cooperative launch (or a few chunks) for all members.  Members are
-// sorted by cells and dealt to chunks in snake order, no chunk holding more than half the
-// blocks that are resident together; a chunk's blocks go to its members in proportion to
-// their cells, at least one each and no more than their tasks fill.
+// sorted by cells and dealt to chunks in snake order; a chunk's blocks go to its members in
+// proportion to their cells, at least one each and no more than their tasks fill.
+//
+// Chunks run one after another, each for as long as its slowest member.  A pass of a member lasts
+// about as long as the rows of its tasks one after another, plus a pass end of some four rows
+// (kEndRows), so between the fewest chunks (a block a member) and twice as many, whose large members
+// have blocks to spare, the count is taken whose chunks' longest passes add up to the least.  Ensemble
+// steps, ms, with the fewest / twice as many chunks: 80 members of sides 8 to 60 1.20 / 1.83, 256 of 8 to
+// 32 2.39 / 3.37, 80 of 64 to 256 12.1 / 9.6, 256 of 64 to 256 60.4 / 37.9.
+constexpr int kEndRows = 4;
 template <class Op, class Job, class K, class Make>
 imex_status add_chunks(BatchSolvePlan* plan, const std::vector<imex_ctx*>& members, K kernel, size_t smem, Make make) {
   imex_ctx* c0 = members[0];
@@ -2090,26 +2097,50 @@ imex_status add_chunks(BatchSolvePlan* plan, const std::vector<imex_ctx*>& membe
   std::vector<int> order(nm);
   for (int m = 0; m < nm; ++m) order[m] = m;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return members[a]->N > members[b]->N; });
-  const int per_chunk = cap / 2 > 0 ? cap / 2 : 1;
-  const int L = (nm + per_chunk - 1) / per_chunk;
-  std::vector<std::vector<int>> groups(L);
-  for (int i = 0; i < nm; ++i) {
-    const int r = i % (2 * L);
-    groups[r < L ? r : 2 * L - 1 - r].push_back(order[i]);
+  auto deal = [&](int L) {
+    std::vector<std::vector<int>> groups(L);
+    for (int i = 0; i < nm; ++i) {
+      const int r = i % (2 * L);
+      groups[r < L ? r : 2 * L - 1 - r].push_back(order[i]);
+    }
+    return groups;
+  };
+  // the cut of every member of a chunk
+  auto cuts = [&](const std::vector<int>& grp) {
+    const int n = (int)grp.size();
+    double cells = 0.0;
+    for (int m : grp) cells += (double)members[m]->N;
+    std::vector<Cut> k;
+    for (int m : grp) k.push_back(make_cut<Op>(members[m], 1 + (int)((double)(cap - n) * (double)members[m]->N / cells)));
+    return k;
+  };
+  std::vector<std::vector<int>> groups;
+  long long least = -1;
+  const int half = cap / 2 > 0 ? cap / 2 : 1;
+  for (int L = (nm + cap - 1) / cap; L <= (nm + half - 1) / half; ++L) {
+    std::vector<std::vector<int>> g = deal(L);
+    long long rows = 0;
+    for (const std::vector<int>& grp : g) {
+      long long slowest = 0;
+      for (const Cut& k : cuts(grp))
+        slowest = std::max(slowest, kEndRows + (long long)((k.per + Op::W - 1) / Op::W) * (k.G.L + 2 * Op::H));
+      rows += slowest;
+    }
+    if (least < 0 || rows < least) {
+      least = rows;
+      groups.swap(g);
+    }
   }
   for (const std::vector<int>& grp : groups) {
     if (grp.empty()) continue;
     const int n = (int)grp.size();
-    double cells = 0.0;
-    for (int m : grp) cells += (double)members[m]->N;
+    const std::vector<Cut> cut = cuts(grp);
     std::vector<Job> jobs;
     std::vector<int> map;
     int first = 0;
     for (int q = 0; q < n; ++q) {
-      imex_ctx* m = members[grp[q]];
-      const int share = 1 + (int)((double)(cap - n) * (double)m->N / cells);
-      const Cut k = make_cut<Op>(m, share);
-      Job j = make(m, k);
+      const Cut& k = cut[q];
+      Job j = make(members[grp[q]], k);
       j.g.first = first;
       jobs.push_back(j);
       for (int u = 0; u < k.nblk; ++u) map.push_back(q);

@@ -156,3 +156,21 @@ def test_batch_solve_tile_shapes_of_the_local_dissipation(tile):
     batch.step(2)
     _check_members(batch, probs, 2, settings, 2, 1e-11, 1e-10)
     batch.close()
+
+
+def test_batch_of_many_small_members_is_one_launch_a_solve():
+    """Eighty small members, more than half the blocks that are resident together: one launch a solve, in which
+    most members have one block, and twice the blocks' number in the launches of two chunks.  Tolerance as above."""
+    probs = [vortex(8 + (7 * m) % 25, 8 + (5 * m) % 23, kappa=0.7 + 0.01 * m) for m in range(80)]
+    batch = ix.Batch(probs, 2, CFG0)
+    batch.step(2)
+    assert batch.info()["solve_launches_per_step"] == 2
+    for m in range(0, 80, 9):
+        single = ix.Solver.for_problem(probs[m], 2, CFG0)
+        single.step()
+        single.step()
+        a, b = batch.members[m].cons(), single.cons()
+        for k in range(8):
+            assert rel(a[k], b[k]) <= 1e-11, (m, k, rel(a[k], b[k]))
+        single.close()
+    batch.close()
