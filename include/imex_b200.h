@@ -137,7 +137,8 @@ typedef struct imex_config {
   double fixed_dt;     /* g_fixed_dt: > 0 forces dt (config.hpp:249) */
   /* additions of this implementation */
   int gmres_restart;      /* Krylov vectors per cycle; the reference hard-codes 25 (implicit_operators.cpp:801) */
-  int gmres_max_restarts; /* restart cap; 0 = the vector dimension, as the reference (implicit_operators.cpp:802) */
+  int gmres_max_restarts; /* restart cap; 0 = the vector dimension, as the reference (implicit_operators.cpp:802).
+                             Conjugate gradients take as many cycles before GMRES goes on with all of its own */
   int precision;          /* imex_precision */
   double mixed_inner_tol; /* relative tolerance of each FP32 inner solve in mixed mode */
   int mixed_max_refine;   /* cap on FP64 refinement sweeps in mixed mode */
