@@ -22,8 +22,8 @@ N ranks each run an independent copy of the workload; value = total
 cell-stage updates of all ranks / max over ranks of the timed span.
 
 --impl reference times the reference solver's own CPU code (oracle/_ref,
-built from the reference sources; else the C restatement) on the host with
-the threads it can use (it is single-threaded), on the same workload and
+built from the reference sources; without it the arm is unavailable) on the host
+with the threads it can use (it is single-threaded), on the same workload and
 grid as the GPU arm.  One of its benchmark steps is one IMEX stage of that
 run (the metric is per stage, and one stage of the 1024^2 vortex sheet takes
 the reference about 13 s on one core), so `--steps K --warmup W` runs W + K
@@ -310,9 +310,13 @@ def run_reference(args, world: int, rank: int) -> None:
     if rank != 0:
         return
     try:
-        import oracle.bindings  # noqa: F401
+        from oracle.bindings import RefSolver
     except Exception as exc:  # pragma: no cover
         print(json.dumps({"impl": "reference", "unavailable": f"oracle import failed: {exc}"}))
+        return
+    if not RefSolver.available():  # the C restatement is this repository's own, no reference to compare with
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not at hand, so its solver "
+                                                              "(oracle/_ref) is not built"}))
         return
     wl = WORKLOADS[args.workload]
     info = host_info()

@@ -82,3 +82,15 @@ def test_reference_stage_stepping_matches_whole_steps():
     assert np.array_equal(whole.cons(), staged.solver.cons())
     assert np.array_equal(whole.vector_potential(), staged.solver.vector_potential())
     assert whole.scalars() == staged.solver.scalars()
+
+
+def test_reference_arm_is_unavailable_without_the_reference(monkeypatch, capsys):
+    """The arm never times this repository's C restatement in the reference's place."""
+    import argparse
+    import json
+    from oracle.bindings import RefSolver
+    monkeypatch.setattr(RefSolver, "available", classmethod(lambda cls: False))
+    bench.run_reference(argparse.Namespace(workload="vortex_sheet_1024", n=16, steps=1, warmup=0, gpus=1,
+                                           precision="fp64", json_out=None), 1, 0)
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
