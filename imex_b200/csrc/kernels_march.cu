@@ -57,6 +57,15 @@ bool supports(const imex_ctx* ctx, int op) {
   if (op == IMEX_OP_MAGNETIC_A) return P.GLF && !P.xclamp && !P.yclamp;
   return P.GLF != 0;
 }
+// The FP64 A form of one small context stays with the tile kernels: a task marches four halo rows beside
+// its two to five, and a pass lasts as long as a task.  us per solve, tile / marching: 64^2 169 / 200, 128^2 154 /
+// 162, 251 x 173 116 / 118, 320^2 138 / 138, 512^2 161 / 127.  The mixed form and ensembles are
+// faster here at every size.
+constexpr size_t kMarchA = 100000;
+bool takes(const imex_ctx* ctx, int op, bool fp64) {
+  if (!supports(ctx, op)) return false;
+  return op != IMEX_OP_MAGNETIC_A || ctx->N >= kMarchA || (!fp64 && is_mixed(ctx, IMEX_MIXED_MAGNETIC));
+}
 imex_status gmres_solve(imex_ctx* ctx, int op, int fam, double* x, const double* b, const Scratch* scratch) {
   const bool rk = ctx->P.eos_type != IMEX_IDEAL_GAS;
   if (op == IMEX_OP_PRESSURE_L || op == IMEX_OP_PRESSURE_J) {

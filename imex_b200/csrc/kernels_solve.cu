@@ -2398,6 +2398,7 @@ long long wait_cycles(const imex_ctx* ctx) {
 }
 imex_status reset_sync(imex_ctx* ctx) {
   k_reset_sync<<<1, 1, 0, ctx->stream>>>(ctx->sync, wait_cycles(ctx));
+  ctx->kernel_launches += 1;
   return cuda_check(ctx, cudaGetLastError(), "sync reset");
 }
 
@@ -2558,7 +2559,7 @@ int gmres_family(int op) {
                                                               : (op == IMEX_OP_ENERGY ? F_GMRES_ENERGY : F_GMRES_PRES));
 }
 imex_status gmres_launch(imex_ctx* ctx, int op, double* x, const double* b) {
-  if (march::supports(ctx, op)) return march::gmres_solve(ctx, op, gmres_family(op), x, b);
+  if (march::takes(ctx, op)) return march::gmres_solve(ctx, op, gmres_family(op), x, b);
   if (op == IMEX_OP_PRESSURE_L || op == IMEX_OP_PRESSURE_J) {
     PressureOp o = make_pressure_op(ctx);
     o.jac = op == IMEX_OP_PRESSURE_J;
@@ -2689,7 +2690,7 @@ imex_status gmres_noalloc_march(imex_ctx* ctx, int op, double* x, const double* 
 // floor slope's inputs min b, max V); 0: the solve reduces them itself
 imex_status newton_launch(imex_ctx* ctx, double* p, const double* b, int keys = 0) {
   const DevParams& P = ctx->P;
-  if (march::supports(ctx, IMEX_OP_PRESSURE_L))
+  if (march::takes(ctx, IMEX_OP_PRESSURE_L))
     return !P.floor_on && P.eos_type == IMEX_IDEAL_GAS ? march::gmres_solve(ctx, IMEX_OP_PRESSURE_L, F_NEWTON, p, b)
                                                        : march::newton_solve(ctx, p, b, keys);
   PressureOp o = make_pressure_op(ctx);
@@ -3188,7 +3189,7 @@ imex_status run_gmres(imex_ctx* ctx, int op, double* x, const double* b) { retur
 
 imex_status run_gmres_noalloc(imex_ctx* ctx, int op, double* x, const double* b, unsigned char* base,
                               size_t capacity) {
-  if (march::supports(ctx, op)) return gmres_noalloc_march(ctx, op, x, b, base, capacity);
+  if (march::takes(ctx, op, true)) return gmres_noalloc_march(ctx, op, x, b, base, capacity);
   if (op == IMEX_OP_PRESSURE_L || op == IMEX_OP_PRESSURE_J) {
     PressureOp o = make_pressure_op(ctx);
     o.jac = op == IMEX_OP_PRESSURE_J;

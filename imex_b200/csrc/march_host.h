@@ -13,8 +13,10 @@ struct Scratch {
   double *V, *AV, *partial;
   SyncState* sync;
 };
-// whether the solve of `op` (imex_op) under this context's configuration runs here
+// whether the solve of `op` (imex_op) under this context's configuration can run here (and does, in an ensemble)
 bool supports(const imex_ctx* ctx, int op);
+// whether one context's solve does; fp64: whatever the configuration's precision (imex_gmres_noalloc)
+bool takes(const imex_ctx* ctx, int op, bool fp64 = false);
 imex_status gmres_solve(imex_ctx* ctx, int op, int fam, double* x, const double* b, const Scratch* scratch = nullptr);
 imex_status newton_solve(imex_ctx* ctx, double* p, const double* b, int keys);
 // the batched solve of every member; nested: the nested Newton instead of the linear pressure solve

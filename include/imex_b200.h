@@ -446,7 +446,7 @@ imex_status imex_divergence(imex_ctx* ctx, double* face_l2, double* cell_wrapped
  * after imex_batch_configure. */
 imex_status imex_set_barrier_timeout(imex_ctx* ctx, double seconds);
 /* Runs `iterations` device-wide barriers of the tile kernels (the solves of the exact
- * arithmetic, the local dissipation and the open A form) with their CTA count and reports
+ * arithmetic, the local dissipation, the open and the small FP64 A form) with their CTA count and reports
  * the mean cost per barrier.  `phantom_blocks` > 0 makes the barrier wait for CTAs
  * that were never launched, so the bounded wait must run out after `timeout_s` and the
  * call must return IMEX_ERR_SYNC (a self-test of the failure path). */

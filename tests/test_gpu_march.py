@@ -341,3 +341,16 @@ def test_mixed_newton_keeps_pressures_above_a_small_floor():
     assert not [s for s in status if s[0] == 0 and s[2] == 7], status
     done = [sum(s[k] == 0 for s in status) for k in range(3)]
     assert done[0] >= 50 and done[2] >= done[1], done
+
+
+@pytest.mark.parametrize("nx,ny,restart", [(393, 255, 25), (4100, 25, 25), (25, 4100, 25), (393, 255, 1), (393, 255, 3),
+                                           (393, 255, 30)])
+def test_march_a_form_of_large_contexts(nx, ny, restart):
+    """The FP64 A form from the 100 thousand cells where one context's solve marches: a strip's width and one column
+    past it, few long and many short runs, Krylov spaces below and past the ring."""
+    sv, prob = _solver("sheet", nx, ny, dict(A_FORM, gmres_restart=restart))
+    sv.prepare_operator("magnetic_A", 2.0 * min(prob.dx, prob.dy))
+    x = _known(sv, "magnetic_A")
+    got, st = sv.gmres("magnetic_A", np.zeros_like(x), sv.apply_operator("magnetic_A", x))
+    assert st["status"] == 0 and rel(got, x) <= 1e-10, (st, rel(got, x))
+    sv.close()
