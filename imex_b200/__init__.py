@@ -660,7 +660,7 @@ class Batch:
                     mixed_solves=t.mixed_solves, solve_tile=(t.solve_tile_x, t.solve_tile_y))
 
     def set_solve_tile(self, tile: int) -> None:
-        """Tile shape of the batched B-form solve (fast arithmetic, local dissipation): 0 = 32x16,
+        """Tile shape of the batched B-form solve (fast arithmetic) where it runs on tiles: 0 = 32x16,
         1 = 64x8, 2 = 32x8 cells; without effect where the marching kernels solve."""
         self._check(self.lib.imex_batch_set_solve_tile(self.b, tile))
 

@@ -554,7 +554,7 @@ imex_status imex_batch_autotune(imex_batch* b, int trial_steps, imex_batch_tunin
   const int solves0 = c0->cfg.mixed_solves;
   const int mag = IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B;
   // the tile shape matters for the B-form solve of the fast arithmetic where the marching kernels do not take it
-  const bool tiles = c0->P.magfield != IMEX_PotentialA && c0->P.fast && !march::supports(c0, IMEX_OP_MAGNETIC_B);
+  const bool tiles = c0->P.magfield != IMEX_PotentialA && c0->P.fast && !march::takes(b->members, IMEX_OP_MAGNETIC_B);
   struct Choice {
     int streams, restart, solves, tile;
   };

@@ -66,6 +66,21 @@ bool takes(const imex_ctx* ctx, int op, bool fp64) {
   if (!supports(ctx, op)) return false;
   return op != IMEX_OP_MAGNETIC_A || ctx->N >= kMarchA || (!fp64 && is_mixed(ctx, IMEX_MIXED_MAGNETIC));
 }
+// Members nearly as many as blocks get one block each here, and the FP64 magnetic solve of one of 32^2 to 64^2
+// cells in one block takes longer than on four tile blocks per SM.  Ensemble steps, ms, B form, tile / marching
+// magnetic solves: 80 members of sides 8 to 60 1.29 / 1.36, 80 of 32 to 64 1.64 / 1.83, 148 of 8 to 60 1.92 / 1.99 (A
+// form 1.76 / 2.08, 2.12 / 2.44, 2.53 / 2.73); 80 of 8 to 24 1.00 / 0.98, 200 of 32 to 64 3.72 / 3.48, 40 of 16 to 64 and
+// the mixed form faster here.
+bool takes(const std::vector<imex_ctx*>& members, int op) {
+  imex_ctx* c0 = members[0];
+  if (!supports(c0, op)) return false;
+  if (op != IMEX_OP_MAGNETIC_A && op != IMEX_OP_MAGNETIC_B) return true;
+  if (is_mixed(c0, op == IMEX_OP_MAGNETIC_A ? IMEX_MIXED_MAGNETIC : IMEX_MIXED_MAGNETIC | IMEX_MIXED_MAGNETIC_B)) return true;
+  const size_t n = members.size(), sms = (size_t)c0->num_sms;
+  size_t largest = 0;
+  for (const imex_ctx* m : members) largest = std::max(largest, m->N);
+  return 2 * n <= sms || n > sms || largest <= 24 * 24 || largest > 64 * 64;
+}
 imex_status gmres_solve(imex_ctx* ctx, int op, int fam, double* x, const double* b, const Scratch* scratch) {
   const bool rk = ctx->P.eos_type != IMEX_IDEAL_GAS;
   if (op == IMEX_OP_PRESSURE_L || op == IMEX_OP_PRESSURE_J) {

@@ -2899,7 +2899,7 @@ imex_status batch_solve_build(const std::vector<imex_ctx*>& members, int kind, B
   imex_status s;
   const int op = kind == BATCH_MAGNETIC ? (P.magfield == IMEX_PotentialA ? IMEX_OP_MAGNETIC_A : IMEX_OP_MAGNETIC_B)
                                         : (P.formula == IMEX_EnergyFormula ? IMEX_OP_ENERGY : IMEX_OP_PRESSURE_L);
-  if (march::supports(c0, op)) {  // members share the configuration
+  if (march::takes(members, op)) {
     s = march::batch_build(plan, members, op, P.floor_on || P.eos_type != IMEX_IDEAL_GAS);
   } else if (kind == BATCH_MAGNETIC) {
     auto sys = [](imex_ctx* m, double** x, const double** b) {

@@ -19,6 +19,8 @@ bool supports(const imex_ctx* ctx, int op);
 bool takes(const imex_ctx* ctx, int op, bool fp64 = false);
 imex_status gmres_solve(imex_ctx* ctx, int op, int fam, double* x, const double* b, const Scratch* scratch = nullptr);
 imex_status newton_solve(imex_ctx* ctx, double* p, const double* b, int keys);
+// whether the batched solve of these members does
+bool takes(const std::vector<imex_ctx*>& members, int op);
 // the batched solve of every member; nested: the nested Newton instead of the linear pressure solve
 imex_status batch_build(BatchSolvePlan* plan, const std::vector<imex_ctx*>& members, int op, bool nested);
 // the same for the Redlich-Kwong gas's pressure solves (kernels_march_rk.cu)

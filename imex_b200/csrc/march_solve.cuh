@@ -2077,16 +2077,18 @@ imex_status newton_one(imex_ctx* ctx, double* p, const double* b, int keys) {
   return s;
 }
 
-// ---- ensembles: one cooperative launch (or a few chunks) for all members.  Members are
-// sorted by cells and dealt to chunks in snake order; a chunk's blocks go to its members in
-// proportion to their cells, at least one each and no more than their tasks fill.
+// ---- ensembles: one cooperative launch (or a few chunks) for all members.  A chunk's blocks go to
+// its members in proportion to their cells, at least one each and no more than their tasks fill.
 //
 // Chunks run one after another, each for as long as its slowest member.  A pass of a member lasts
 // about as long as the rows of its tasks one after another, plus a pass end of some four rows
-// (kEndRows), so between the fewest chunks (a block a member) and twice as many, whose large members
-// have blocks to spare, the count is taken whose chunks' longest passes add up to the least.  Ensemble
-// steps, ms, with the fewest / twice as many chunks: 80 members of sides 8 to 60 1.20 / 1.83, 256 of 8 to
-// 32 2.39 / 3.37, 80 of 64 to 256 12.1 / 9.6, 256 of 64 to 256 60.4 / 37.9.
+// (kEndRows).  Members are sorted by cells, and of the ways to cut their order into chunks of at most
+// a block each (at every 24th of the members) the one is taken whose chunks' longest passes add up to
+// the least: small members share a launch, a block each, and large ones have blocks to spare.  Ensemble
+// steps, ms, tile kernels / chunks of half the blocks, dealt in turn / cut like this:
+// 256 members of sides 64 to 256 35.1 / 38.0 / 24.4, 80 of 64 to 256 9.9 / 9.5 / 8.0, 256 of 16 to 64 4.41 /
+// 5.10 / 3.61, 400 of 16 to 64 6.31 / 7.94 / 5.25, 80 of 8 to 60 1.22 / 1.84 / 1.33, 150 of 8 to 60 2.05 / 2.90 /
+// 2.28.
 constexpr int kEndRows = 4;
 template <class Op, class Job, class K, class Make>
 imex_status add_chunks(BatchSolvePlan* plan, const std::vector<imex_ctx*>& members, K kernel, size_t smem, Make make) {
@@ -2097,14 +2099,6 @@ imex_status add_chunks(BatchSolvePlan* plan, const std::vector<imex_ctx*>& membe
   std::vector<int> order(nm);
   for (int m = 0; m < nm; ++m) order[m] = m;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return members[a]->N > members[b]->N; });
-  auto deal = [&](int L) {
-    std::vector<std::vector<int>> groups(L);
-    for (int i = 0; i < nm; ++i) {
-      const int r = i % (2 * L);
-      groups[r < L ? r : 2 * L - 1 - r].push_back(order[i]);
-    }
-    return groups;
-  };
   // the cut of every member of a chunk
   auto cuts = [&](const std::vector<int>& grp) {
     const int n = (int)grp.size();
@@ -2114,23 +2108,34 @@ imex_status add_chunks(BatchSolvePlan* plan, const std::vector<imex_ctx*>& membe
     for (int m : grp) k.push_back(make_cut<Op>(members[m], 1 + (int)((double)(cap - n) * (double)members[m]->N / cells)));
     return k;
   };
-  std::vector<std::vector<int>> groups;
-  long long least = -1;
-  const int half = cap / 2 > 0 ? cap / 2 : 1;
-  for (int L = (nm + cap - 1) / cap; L <= (nm + half - 1) / half; ++L) {
-    std::vector<std::vector<int>> g = deal(L);
+  auto slowest = [&](int from, int to) {
     long long rows = 0;
-    for (const std::vector<int>& grp : g) {
-      long long slowest = 0;
-      for (const Cut& k : cuts(grp))
-        slowest = std::max(slowest, kEndRows + (long long)((k.per + Op::W - 1) / Op::W) * (k.G.L + 2 * Op::H));
-      rows += slowest;
+    for (const Cut& k : cuts(std::vector<int>(order.begin() + from, order.begin() + to)))
+      rows = std::max(rows, kEndRows + (long long)((k.per + Op::W - 1) / Op::W) * (k.G.L + 2 * Op::H));
+    return rows;
+  };
+  const int step = std::max(1, std::min(nm / 24, cap));
+  std::vector<int> at;  // where a chunk may end
+  for (int i = 0; i < nm; i += step) at.push_back(i);
+  if (nm > cap) at.push_back(nm - cap);
+  at.push_back(nm);
+  std::sort(at.begin(), at.end());
+  const int np = (int)at.size();
+  std::vector<long long> least(np, -1);  // rows of the chunks up to there, and where the last one begins
+  std::vector<int> begin(np, 0);
+  least[0] = 0;
+  for (int e = 1; e < np; ++e)
+    for (int a = 0; a < e; ++a) {
+      if (at[e] - at[a] > cap || least[a] < 0) continue;
+      const long long rows = least[a] + (at[e] > at[a] ? slowest(at[a], at[e]) : 0);
+      if (least[e] < 0 || rows < least[e]) {
+        least[e] = rows;
+        begin[e] = a;
+      }
     }
-    if (least < 0 || rows < least) {
-      least = rows;
-      groups.swap(g);
-    }
-  }
+  std::vector<std::vector<int>> groups;
+  for (int e = np - 1; e > 0; e = begin[e])
+    groups.insert(groups.begin(), std::vector<int>(order.begin() + at[begin[e]], order.begin() + at[e]));
   for (const std::vector<int>& grp : groups) {
     if (grp.empty()) continue;
     const int n = (int)grp.size();

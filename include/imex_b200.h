@@ -415,10 +415,10 @@ imex_status imex_batch_step(imex_batch* b, int steps, double* device_ms);
  * batched solves (a cooperative launch per chunk, with a barrier reset before it in the tile
  * kernels); -1 in the streams mode.  The second pointer may be null. */
 imex_status imex_batch_explicit_launches(imex_batch* b, int* launches_per_step, int* solve_launches_per_step);
-/* tile shape of the batched B-form magnetic solve in the fast arithmetic with local dissipation
- * (GLF = 0): 0 = 32 x 16 cells (the default, and the shape of every single-context tile solve),
- * 1 = 64 x 8, 2 = 32 x 8.  Without effect where the row-marching kernels solve (GLF = 1), which
- * have no tiles. */
+/* tile shape of the batched B-form magnetic solve in the fast arithmetic where it runs on tiles (local
+ * dissipation, GLF = 0, and FP64 ensembles of about as many small members as SMs): 0 = 32 x 16 cells (the
+ * default, and the shape of every single-context tile solve), 1 = 64 x 8, 2 = 32 x 8.  Without
+ * effect where the row-marching kernels solve, which have no tiles. */
 imex_status imex_batch_set_solve_tile(imex_batch* b, int tile);
 /* time `trial_steps` ensemble steps per candidate, one choice at a time from the best so
  * far: the explicit mode (batched launches, or 4 / 8 / 16 streams), the B-form solve's tile

@@ -158,10 +158,12 @@ def test_batch_solve_tile_shapes_of_the_local_dissipation(tile):
     batch.close()
 
 
-def test_batch_of_many_small_members_is_one_launch_a_solve():
+@pytest.mark.parametrize("longest", [24, 40])
+def test_batch_of_many_small_members_is_one_launch_a_solve(longest):
     """Eighty small members, more than half the blocks that are resident together: one launch a solve, in which
-    most members have one block, and twice the blocks' number in the launches of two chunks.  Tolerance as above."""
-    probs = [vortex(8 + (7 * m) % 25, 8 + (5 * m) % 23, kappa=0.7 + 0.01 * m) for m in range(80)]
+    most members have one block (to 24^2 cells all solves march, from there the FP64 magnetic ones run on tiles).
+    Tolerance as above."""
+    probs = [vortex(8 + (7 * m) % (longest - 7), 8 + (5 * m) % (longest - 7), kappa=0.7 + 0.01 * m) for m in range(80)]
     batch = ix.Batch(probs, 2, CFG0)
     batch.step(2)
     assert batch.info()["solve_launches_per_step"] == 2
@@ -172,5 +174,25 @@ def test_batch_of_many_small_members_is_one_launch_a_solve():
         a, b = batch.members[m].cons(), single.cons()
         for k in range(8):
             assert rel(a[k], b[k]) <= 1e-11, (m, k, rel(a[k], b[k]))
+        single.close()
+    batch.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_batch_of_more_members_than_blocks(precision):
+    """Uneven members in several launches a solve, cut at the ensemble's own places: 160 of sides 4 to 60, whose
+    largest and smallest share no launch.  Mixed solves stop at 1e-10."""
+    probs = [vortex(4 + (37 * m) % 57, 4 + (23 * m) % 57, kappa=0.7 + 0.005 * m) for m in range(160)]
+    settings = dict(CFG0, precision=precision)
+    batch = ix.Batch(probs, 2, settings)
+    batch.step(2)
+    assert batch.info()["solve_launches_per_step"] >= 4
+    for m in range(0, 160, 13):
+        single = ix.Solver.for_problem(probs[m], 2, settings)
+        single.step()
+        single.step()
+        a, b = batch.members[m].cons(), single.cons()
+        for k in range(8):
+            assert rel(a[k], b[k]) <= (1e-11 if precision == "fp64" else 1e-8), (m, k, rel(a[k], b[k]))
         single.close()
     batch.close()
